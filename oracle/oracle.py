@@ -36,7 +36,7 @@ class oracle_params(C.Structure):
 def build(quiet=True):
     """Compile the oracles (O1 only where the reference sources are present)."""
     targets = ["_ref/liboracle.so"]
-    if os.path.isdir(REFERENCE_SRC):
+    if os.path.isfile(os.path.join(REFERENCE_SRC, "src", "System", "PBC.cpp")):
         targets.append("_ref/o1_harness")
         # the reference's own System on libmdf (needs libmdf.so built first)
         if os.path.exists(os.path.join(os.path.dirname(HERE), "md_b200", "libmdf.so")):
