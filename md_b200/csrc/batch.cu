@@ -211,6 +211,7 @@ struct MultiArgs {
     size_t dyn_pairs = 0;
     int threads = 256;
     bool prune_on = false, use_switch = false, energy = false, persist = false, half = false;
+    bool parts = false;    // some system's lists are cut into parts
     bool lj_smem = true;   // every system's LJ table in shared memory (one kernel form for the batch)
 };
 
@@ -330,6 +331,13 @@ MultiDev<R> prepare_multi(mdf_batch* b, uint32_t flags, MultiArgs<R>& M, double*
         for (auto& a : M.p64) a.lj_smem = 0;
         M.dyn_pairs = 0;
     }
+    // shares of the pair lists: by the work of the whole batch
+    long long nlist = 0;
+    for (const auto& a : M.pf32) nlist += a.nlist;
+    for (auto& a : M.pf32) {
+        set_pair_split(a, pair_split(nlist), M.threads / 32);
+        M.parts = M.parts || a.part < WHOLE_LIST;
+    }
     M.gx_prune = gmax(M.prune);
     M.gx_pairs = sizeof(R) == 4 ? gmax(M.pf32) : gmax(M.p64);
     M.gx_excl = gmax(M.excl);
@@ -432,7 +440,7 @@ void enqueue_multi(mdf_batch* b, const MultiArgs<R>& M, const MultiDev<R>& D, co
     if (M.gx_pairs > 0) {
         if (sizeof(R) == 4)
             launch_pairs_f32_multi(D.pf32, n, M.gx_pairs, M.threads, M.dyn_pairs, M.energy, M.use_switch, M.persist,
-                                   M.half, M.lj_smem, b->main);
+                                   M.half, M.lj_smem, M.parts, b->main);
         else
             launch_pairs_f64_multi(D.p64, n, M.gx_pairs, M.threads, M.dyn_pairs, M.energy, M.use_switch, M.persist,
                                    M.half, M.lj_smem, b->main);

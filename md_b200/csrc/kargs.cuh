@@ -70,6 +70,8 @@ struct PruneArgs {
 };
 
 // ------------------------------------------------------------- pair kernels
+constexpr int WHOLE_LIST = 1 << 30;   // a list is one part (PairF32Args::part)
+
 // Constants of the FP32 pair kernel, folded on the host.
 struct PairConstF {
     float rc2;
@@ -101,7 +103,9 @@ struct PairF32Args {
     unsigned long long* npairs;
     unsigned long long* next;   // work counter of the persistent warps, zero at launch
     int persist;                // 1: persistent warps on the counter; 0: warp w takes item w
-    int half;                   // items are half entries (the 4 x 8 kernel)
+    int half;                   // lists are half entries (the 4 x 8 kernel)
+    int split;                  // log2 of the shares (items) each list is cut into
+    int part;                   // entries per part (pair_part), or WHOLE_LIST
     unsigned* st;
 };
 
@@ -137,7 +141,7 @@ struct PairF64Args {
     unsigned long long* npairs;
     unsigned long long* next;   // work counter of the persistent warps, zero at launch
     int persist;                // 1: persistent warps on the counter; 0: warp w takes item w
-    int half;                   // items are half entries (the 4 x 8 kernel)
+    int half;                   // lists are half entries (the 4 x 8 kernel)
     unsigned* st;
 };
 
@@ -355,12 +359,19 @@ template <typename R>
 void launch_prune_multi(const PruneArgs<R>* d_args, int nsys, int gx, bool half, cudaStream_t s);
 PairF32Args make_pair_f32_args(const Ctx& c, size_t* dyn);
 void launch_pairs_f32_multi(const PairF32Args* d_args, int nsys, int gx, int threads, size_t dyn, bool energy,
-                            bool use_switch, bool persist, bool half, bool lj_smem, cudaStream_t s);
+                            bool use_switch, bool persist, bool half, bool lj_smem, bool parts, cudaStream_t s);
 template <typename R> PairArgs<R> make_pair_args(const Ctx& c, bool count);
 PairF64Args make_pair_f64_args(const Ctx& c, size_t* dyn);
 void launch_pairs_f64_multi(const PairF64Args* d_args, int nsys, int gx, int threads, size_t dyn, bool energy,
                             bool use_switch, bool persist, bool half, bool lj_smem, cudaStream_t s);
 int pair_threads(const Ctx& c);
+int pair_split(long long nlist);
+// 2^split items per list, one warp each.
+inline void set_pair_split(PairF32Args& a, int split, int warps_per_block)
+{
+    a.split = a.part < WHOLE_LIST ? split : 0;
+    a.gx = grid_blocks((long long)a.nlist << a.split, warps_per_block);
+}
 ExclArgs make_excl_args(const Ctx& c);
 Pair14Args make_pair14_args(const Ctx& c);
 void launch_exclusions_multi(const ExclArgs* d_excl, int gx_excl, const Pair14Args* d_14, int gx_14, int nsys,

@@ -286,6 +286,33 @@ __global__ void __launch_bounds__(NB_THREADS) k_pairs_multi(const PairArgs<R>* _
 //  * each lane loads its entry of the next batch of four one batch ahead;
 //  * energies are summed in FP32 per entry and in FP64 across entries.
 
+// ------------------------------------------------------ shares of a list
+// A warp's item is one of 2^split shares of an i cluster's list.  Lists of
+// systems below SPLIT_CLUSTERS clusters are cut into parts of PART_ENTRIES
+// entries: i forces and energies are reduced over the lanes and added in fixed
+// point at the end of every part, and a share holds whole parts, so the split
+// (a launch shape) changes no bit; in larger systems a list is one part and
+// one item.  Without shares the warp of an i cluster walks its ~70 entries
+// alone and leaves the chip idle: pair launch (forces) 43 -> 17 us at 887
+// atoms, 56 -> 20 at 2,780, 50 -> 30 at 6,398, 57 -> 38 at 12,101 (evaluation
+// 129 -> 94 us there).  At 28,000 atoms (3,241 clusters) two shares took the
+// launch from 67 to 60 us but the evaluation from 160 to 162, its side stream
+// filling the SMs the fewer warps leave: the line lies below that.  The parts'
+// reductions cost a batch of small systems, which needs no shares, 1.4% (16
+// entries per part 2.1%, 32 1.0% but 10-20% on the launches above).
+constexpr int PART_ENTRIES = 24;
+constexpr int SPLIT_CLUSTERS = 2048;
+
+__device__ __forceinline__ void item_range(int count, int item, int split, int& b0, int& b1)
+{
+    b0 = 0;
+    b1 = count;
+    if (split == 0) return;
+    const int parts = (count + PART_ENTRIES - 1) / PART_ENTRIES, s = item & ((1 << split) - 1);
+    b0 = ((parts * s) >> split) * PART_ENTRIES;
+    b1 = min(count, ((parts * (s + 1)) >> split) * PART_ENTRIES);
+}
+
 // Static shared arrays of the pair bodies, declared once per kernel (each
 // kernel inlines two forms of its body, see pairs_f32_body).
 struct SmemF32W {
@@ -309,13 +336,13 @@ struct SmemF64H {
     double sh[27][3];
 };
 
-template <bool ENERGY, bool SWITCH, bool COUNT, bool LJS>
+template <bool ENERGY, bool SWITCH, bool COUNT, bool LJS, bool PARTS>
 __device__ __forceinline__ void pairs_f32_body_t(SmemF32W& S,
     int nlist, const ILRange* __restrict__ ilist, const PairEntry* __restrict__ plist, const float4* __restrict__ xq,
     const int* __restrict__ stype, const float4* __restrict__ centerf, const float4* __restrict__ lj4, int ntp,
     int lj_smem, float kc, const PairConstF& Kin, const ShiftTable& shifts, unsigned long long* __restrict__ fslot,
     int nslots, unsigned long long* __restrict__ acc, unsigned long long* __restrict__ npairs,
-    unsigned long long* __restrict__ next, int persist, unsigned* st)
+    unsigned long long* __restrict__ next, int persist, int split, int part, unsigned* st)
 {
     const PairConstF K = Kin;   // registers (the multi-system launch reads it from device memory)
     extern __shared__ float4 s_lj[];
@@ -334,11 +361,12 @@ __device__ __forceinline__ void pairs_f32_body_t(SmemF32W& S,
     const int jslot = lane >> 3, ii = lane & 7;
     const unsigned FULL = 0xffffffffu;
     int npc = 0;
-    // persist: persistent warps, each taking the next i cluster from the work
+    // An item is one of the 2^split shares of an i cluster's list (item_range).
+    // persist: persistent warps, each taking the next item from the work
     // counter until the list is done (no SM idles behind a slow block or a
-    // partial last wave); otherwise warp w takes i cluster w.  Energies go to
-    // fixed point once per i cluster (a fixed-order FP64 sum), so they do not
-    // depend on which warp took which cluster.
+    // partial last wave); otherwise warp w takes item w.  i forces and energies
+    // go to fixed point once per part (fixed-order sums), so they depend
+    // neither on the split nor on which warp took which item.
     for (int round = 0;; ++round) {
         int w = 0;
         if (persist) {
@@ -348,10 +376,11 @@ __device__ __forceinline__ void pairs_f32_body_t(SmemF32W& S,
             if (round) break;
             w = blockIdx.x * (blockDim.x >> 5) + wib;
         }
-        if (w >= nlist) break;
-        double e_lj = 0, e_dir = 0;
-        float fix = 0.f, fiy = 0.f, fiz = 0.f;
-        const ILRange L = ilist[w];
+        if (w >= (PARTS ? nlist << split : nlist)) break;
+        const ILRange L = ilist[PARTS ? w >> split : w];
+        int b0 = 0, b1 = L.count;
+        if (PARTS) item_range(L.count, w, split, b0, b1);
+        if (b0 >= b1) continue;
         const int I = L.i;
         const float4 xi = xq[I * CLUSTER + ii];
         const int trow = stype[I * CLUSTER + ii] * ntp * (int)sizeof(float4);   // byte offsets
@@ -361,108 +390,115 @@ __device__ __forceinline__ void pairs_f32_body_t(SmemF32W& S,
         const int rot_src = (lane & ~7) | ((ii + 1) & 7);
         // the lane's entry of the next batch is loaded one batch ahead
         PairEntry pn;
-        if (jslot < L.count) {
-            pn = plist[L.start + jslot];
+        if (b0 + jslot < b1) {
+            pn = plist[L.start + b0 + jslot];
         } else {
             pn.j = I; pn.shift = 13; pn.mask = 0ull;
         }
-        for (int b = 0; b < L.count; b += 4) {
-            const int e = b + jslot;
-            const PairEntry pe = pn;
-            if (e + 4 < L.count) {
-                pn = plist[L.start + e + 4];
-            } else {
-                pn.j = I; pn.shift = 13; pn.mask = 0ull;
-            }
-            const int J = pe.j;
-            const float4 xjj = xq[J * CLUSTER + ii];
-            const int tjj = stype[J * CLUSTER + ii] * (int)sizeof(float4);
-            sx[wib][jslot][ii] = xjj;
-            sx[wib][jslot][ii + CLUSTER] = xjj;
-            stj[wib][jslot][ii] = tjj;
-            stj[wib][jslot][ii + CLUSTER] = tjj;
-            const float4 cJ = centerf[J];
-            const float* s6 = sh[pe.shift];
-            const float xix = xi.x + (((cI.x - cJ.x) - s6[0]) - s6[3]);
-            const float xiy = xi.y + (((cI.y - cJ.y) - s6[1]) - s6[4]);
-            const float xiz = xi.z + (((cI.z - cJ.z) - s6[2]) - s6[5]);
-            const unsigned rowm = (unsigned)(pe.mask >> (ii * 8)) & 0xffu;
-            const unsigned rot = ((rowm >> ii) | (rowm << (8 - ii))) & 0xffu;
-            __syncwarp();
-            float fjx = 0.f, fjy = 0.f, fjz = 0.f, el = 0.f, ed = 0.f;
-            const float4* __restrict__ sxl = &sx[wib][jslot][ii];
-            const int* __restrict__ stl = &stj[wib][jslot][ii];
-#pragma unroll
-            for (int t = 0; t < CLUSTER; ++t) {
-                const float4 xj = sxl[t];
-                const float dx = xix - xj.x, dy = xiy - xj.y, dz = xiz - xj.z;
-                const float r2r = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                const bool on = ((rot >> t) & 1u) && r2r <= K.rc2;
-                // switched LJ: a slot outside the list or the cutoff takes r^2 = 1e30,
-                // at which every term below is exactly zero (r^-6 underflows, the
-                // Gaussian is 0 and the switch is 0 at x = 1), so no result needs a select
-                const float r2 = SWITCH ? (on ? r2r : 1e30f) : r2r;
-                const float rinv = rsqrt_ftz(r2);
-                const float r = r2 * rinv, rinv2 = rinv * rinv, rinv6 = rinv2 * rinv2 * rinv2;
-                const float4 ab = at_bytes(ljt, trow + stl[t]);      // A, B, 12A, 6B
-                float U = rinv6 * fmaf(ab.x, rinv6, -ab.y);
-                float G = (rinv6 * rinv2) * fmaf(ab.z, rinv6, -ab.w);
-                if (SWITCH) {
-                    const float x = __saturatef(fmaf(r, K.inv_sw, -K.rsw_inv)), x2 = x * x;
-                    const float S = fmaf(x2 * x, fmaf(x, fmaf(x, -6.f, 15.f), -10.f), 1.f);
-                    const float dSr = x2 * fmaf(x, fmaf(x, K.d30, K.d60), K.d30) * rinv;   // dS/dr / r
-                    G = fmaf(S, G, -U * dSr);
-                    U = U * S;
+        int p = b0;
+        do {
+            const int pe1 = PARTS ? min(p + part, b1) : b1;
+            double e_lj = 0, e_dir = 0;
+            float fix = 0, fiy = 0, fiz = 0;
+            for (int b = p; b < pe1; b += 4) {
+                const int e = b + jslot;
+                const PairEntry pe = pn;
+                if (e + 4 < b1) {
+                    pn = plist[L.start + e + 4];
                 } else {
-                    const float uc = ab.x * K.uc12 - ab.y * K.uc6;
-                    const float gc = (ab.z * K.uc12 - ab.w * K.uc6) / K.rc2f;
-                    U = U - uc + (r - K.rcf) * (gc * K.rcf);
-                    G = G - gc * K.rcf * rinv;
+                    pn.j = I; pn.shift = 13; pn.mask = 0ull;
                 }
-                const float ex = ex2_approx(K.kex * r2);
-                const float erfcv = erfc_as(rcp_ftz(fmaf(K.pa, r, 1.0f)), ex);
-                const float ec = (qik * xj.w) * erfcv * rinv;
-                float g = fmaf(fmaf(qik2 * xj.w, ex, ec), rinv2, G);
-                if (!SWITCH) g = on ? g : 0.f;
+                const int J = pe.j;
+                const float4 xjj = xq[J * CLUSTER + ii];
+                const int tjj = stype[J * CLUSTER + ii] * (int)sizeof(float4);
+                sx[wib][jslot][ii] = xjj;
+                sx[wib][jslot][ii + CLUSTER] = xjj;
+                stj[wib][jslot][ii] = tjj;
+                stj[wib][jslot][ii + CLUSTER] = tjj;
+                const float4 cJ = centerf[J];
+                const float* s6 = sh[pe.shift];
+                const float xix = xi.x + (((cI.x - cJ.x) - s6[0]) - s6[3]);
+                const float xiy = xi.y + (((cI.y - cJ.y) - s6[1]) - s6[4]);
+                const float xiz = xi.z + (((cI.z - cJ.z) - s6[2]) - s6[5]);
+                const unsigned rowm = (unsigned)(pe.mask >> (ii * 8)) & 0xffu;
+                const unsigned rot = ((rowm >> ii) | (rowm << (8 - ii))) & 0xffu;
+                __syncwarp();
+                float fjx = 0.f, fjy = 0.f, fjz = 0.f, el = 0.f, ed = 0.f;
+                const float4* __restrict__ sxl = &sx[wib][jslot][ii];
+                const int* __restrict__ stl = &stj[wib][jslot][ii];
+#pragma unroll
+                for (int t = 0; t < CLUSTER; ++t) {
+                    const float4 xj = sxl[t];
+                    const float dx = xix - xj.x, dy = xiy - xj.y, dz = xiz - xj.z;
+                    const float r2r = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                    const bool on = ((rot >> t) & 1u) && r2r <= K.rc2;
+                    // switched LJ: a slot outside the list or the cutoff takes r^2 = 1e30,
+                    // at which every term below is exactly zero (r^-6 underflows, the
+                    // Gaussian is 0 and the switch is 0 at x = 1), so no result needs a select
+                    const float r2 = SWITCH ? (on ? r2r : 1e30f) : r2r;
+                    const float rinv = rsqrt_ftz(r2);
+                    const float r = r2 * rinv, rinv2 = rinv * rinv, rinv6 = rinv2 * rinv2 * rinv2;
+                    const float4 ab = at_bytes(ljt, trow + stl[t]);      // A, B, 12A, 6B
+                    float U = rinv6 * fmaf(ab.x, rinv6, -ab.y);
+                    float G = (rinv6 * rinv2) * fmaf(ab.z, rinv6, -ab.w);
+                    if (SWITCH) {
+                        const float x = __saturatef(fmaf(r, K.inv_sw, -K.rsw_inv)), x2 = x * x;
+                        const float S = fmaf(x2 * x, fmaf(x, fmaf(x, -6.f, 15.f), -10.f), 1.f);
+                        const float dSr = x2 * fmaf(x, fmaf(x, K.d30, K.d60), K.d30) * rinv;   // dS/dr / r
+                        G = fmaf(S, G, -U * dSr);
+                        U = U * S;
+                    } else {
+                        const float uc = ab.x * K.uc12 - ab.y * K.uc6;
+                        const float gc = (ab.z * K.uc12 - ab.w * K.uc6) / K.rc2f;
+                        U = U - uc + (r - K.rcf) * (gc * K.rcf);
+                        G = G - gc * K.rcf * rinv;
+                    }
+                    const float ex = ex2_approx(K.kex * r2);
+                    const float erfcv = erfc_as(rcp_ftz(fmaf(K.pa, r, 1.0f)), ex);
+                    const float ec = (qik * xj.w) * erfcv * rinv;
+                    float g = fmaf(fmaf(qik2 * xj.w, ex, ec), rinv2, G);
+                    if (!SWITCH) g = on ? g : 0.f;
+                    if (ENERGY) {
+                        el += SWITCH ? U : (on ? U : 0.f);
+                        ed += SWITCH ? ec : (on ? ec : 0.f);
+                    }
+                    if (COUNT) npc += on ? 1 : 0;
+                    fix = fmaf(g, dx, fix); fiy = fmaf(g, dy, fiy); fiz = fmaf(g, dz, fiz);
+                    fjx = fmaf(-g, dx, fjx); fjy = fmaf(-g, dy, fjy); fjz = fmaf(-g, dz, fjz);
+                    fjx = __shfl_sync(FULL, fjx, rot_src);
+                    fjy = __shfl_sync(FULL, fjy, rot_src);
+                    fjz = __shfl_sync(FULL, fjz, rot_src);
+                }
                 if (ENERGY) {
-                    el += SWITCH ? U : (on ? U : 0.f);
-                    ed += SWITCH ? ec : (on ? ec : 0.f);
+                    e_lj += (double)el;
+                    e_dir += (double)ed;
                 }
-                if (COUNT) npc += on ? 1 : 0;
-                fix = fmaf(g, dx, fix); fiy = fmaf(g, dy, fiy); fiz = fmaf(g, dz, fiz);
-                fjx = fmaf(-g, dx, fjx); fjy = fmaf(-g, dy, fjy); fjz = fmaf(-g, dz, fjz);
-                fjx = __shfl_sync(FULL, fjx, rot_src);
-                fjy = __shfl_sync(FULL, fjy, rot_src);
-                fjz = __shfl_sync(FULL, fjz, rot_src);
+                if (e < b1 && (fjx != 0.f || fjy != 0.f || fjz != 0.f)) {
+                    const int sl = J * CLUSTER + ii;
+                    fx_add_force_f(fslot + sl, fjx, st);
+                    fx_add_force_f(fslot + nslots + sl, fjy, st);
+                    fx_add_force_f(fslot + 2 * nslots + sl, fjz, st);
+                }
+                __syncwarp();
+            }
+            fix += __shfl_xor_sync(FULL, fix, 8); fix += __shfl_xor_sync(FULL, fix, 16);
+            fiy += __shfl_xor_sync(FULL, fiy, 8); fiy += __shfl_xor_sync(FULL, fiy, 16);
+            fiz += __shfl_xor_sync(FULL, fiz, 8); fiz += __shfl_xor_sync(FULL, fiz, 16);
+            if (jslot == 0) {
+                const int sl = I * CLUSTER + ii;
+                fx_add_force_f(fslot + sl, fix, st);
+                fx_add_force_f(fslot + nslots + sl, fiy, st);
+                fx_add_force_f(fslot + 2 * nslots + sl, fiz, st);
             }
             if (ENERGY) {
-                e_lj += (double)el;
-                e_dir += (double)ed;
+                const double s_lj = warp_sum(e_lj), s_dir = warp_sum(e_dir);
+                if (lane == 0) {
+                    if (s_lj != 0.0) fx_add(acc + MDF_E_VDW, s_lj, ENERGY_SCALE, st);
+                    if (s_dir != 0.0) fx_add(acc + MDF_E_EE_DIRECT, s_dir, ENERGY_SCALE, st);
+                }
             }
-            if (e < L.count && (fjx != 0.f || fjy != 0.f || fjz != 0.f)) {
-                const int sl = J * CLUSTER + ii;
-                fx_add_force_f(fslot + sl, fjx, st);
-                fx_add_force_f(fslot + nslots + sl, fjy, st);
-                fx_add_force_f(fslot + 2 * nslots + sl, fjz, st);
-            }
-            __syncwarp();
-        }
-        fix += __shfl_xor_sync(FULL, fix, 8); fix += __shfl_xor_sync(FULL, fix, 16);
-        fiy += __shfl_xor_sync(FULL, fiy, 8); fiy += __shfl_xor_sync(FULL, fiy, 16);
-        fiz += __shfl_xor_sync(FULL, fiz, 8); fiz += __shfl_xor_sync(FULL, fiz, 16);
-        if (jslot == 0) {
-            const int sl = I * CLUSTER + ii;
-            fx_add_force_f(fslot + sl, fix, st);
-            fx_add_force_f(fslot + nslots + sl, fiy, st);
-            fx_add_force_f(fslot + 2 * nslots + sl, fiz, st);
-        }
-        if (ENERGY) {
-            const double s_lj = warp_sum(e_lj), s_dir = warp_sum(e_dir);
-            if (lane == 0) {
-                if (s_lj != 0.0) fx_add(acc + MDF_E_VDW, s_lj, ENERGY_SCALE, st);
-                if (s_dir != 0.0) fx_add(acc + MDF_E_EE_DIRECT, s_dir, ENERGY_SCALE, st);
-            }
-        }
+            p = pe1;
+        } while (PARTS && p < b1);
     }
     if (COUNT) {
         long long np = warp_sum_ll((long long)npc);
@@ -482,7 +518,7 @@ __device__ __forceinline__ void pairs_f32_body_t(SmemF32W& S,
 // rotate one lane per step (the lane's i atom repeats every four lanes, so
 // the same shuffle as the whole-entry kernel works).  After the item the
 // eight partial sums of each i atom are reduced by three butterfly steps.
-template <bool ENERGY, bool SWITCH, bool COUNT, bool LJS>
+template <bool ENERGY, bool SWITCH, bool COUNT, bool LJS, bool PARTS>
 __device__ __forceinline__ void pairs_f32_half_body_t(SmemF32H& S, const PairF32Args& A)
 {
     extern __shared__ float4 s_lj[];
@@ -517,8 +553,12 @@ __device__ __forceinline__ void pairs_f32_half_body_t(SmemF32H& S, const PairF32
             if (round) break;
             w = blockIdx.x * (blockDim.x >> 5) + wib;
         }
-        if (w >= nlist) break;
-        const ILRange L = ilist[w];
+        if (w >= (PARTS ? nlist << A.split : nlist)) break;
+        const ILRange L = ilist[PARTS ? w >> A.split : w];
+        const int part = A.part;
+        int b0 = 0, b1 = L.count;
+        if (PARTS) item_range(L.count, w, A.split, b0, b1);
+        if (b0 >= b1) continue;
         const int I = L.i, h = L.pad;
         if (lane < 8) {
             float4 v = xq[I * CLUSTER + 4 * h + (lane & 3)];
@@ -530,106 +570,114 @@ __device__ __forceinline__ void pairs_f32_half_body_t(SmemF32H& S, const PairF32
         const float4 cI = centerf[I];
         const float4* __restrict__ sxl = &sxi[wib][i4];
         const int* __restrict__ stl = &sti[wib][i4];
-        double e_lj = 0, e_dir = 0;
-        float fix = 0.f, fiy = 0.f, fiz = 0.f;   // the i atom (jj + t) & 3 at step t
         // the lane's entry of the next batch is loaded one batch ahead
         PairEntry pn;
-        if (eslot < L.count) {
-            pn = plist[L.start + eslot];
+        if (b0 + eslot < b1) {
+            pn = plist[L.start + b0 + eslot];
         } else {
             pn.j = I; pn.shift = 13; pn.mask = 0ull;
         }
-        for (int b = 0; b < L.count; b += 4) {
-            const int e = b + eslot;
-            const PairEntry pe = pn;
-            if (e + 4 < L.count) {
-                pn = plist[L.start + e + 4];
-            } else {
-                pn.j = I; pn.shift = 13; pn.mask = 0ull;
-            }
-            const int J = pe.j;
-            const float4 xj = xq[J * CLUSTER + jj];
-            const int tj = stype[J * CLUSTER + jj] * (int)sizeof(float4);
-            const float4 cJ = centerf[J];
-            const float* s6 = sh[pe.shift];
-            // the j atom in I's frame: x_j - D, D = (c_I - c_J) - image offset
-            const float pjx = xj.x - (((cI.x - cJ.x) - s6[0]) - s6[3]);
-            const float pjy = xj.y - (((cI.y - cJ.y) - s6[1]) - s6[4]);
-            const float pjz = xj.z - (((cI.z - cJ.z) - s6[2]) - s6[5]);
-            // mask bits (4h + i) * 8 + jj, i = 0..3, rotated so step t tests bit t
-            const unsigned long long mc = pe.mask >> (32 * h + jj);
-            const unsigned nib = (unsigned)((mc & 1ull) | ((mc >> 7) & 2ull) | ((mc >> 14) & 4ull) | ((mc >> 21) & 8ull));
-            const unsigned rot = ((nib >> i4) | (nib << (4 - i4))) & 0xfu;
-            float fjx = 0.f, fjy = 0.f, fjz = 0.f, el = 0.f, ed = 0.f;
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const float4 xi = sxl[t];
-                const float dx = xi.x - pjx, dy = xi.y - pjy, dz = xi.z - pjz;
-                const float r2r = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                const bool on = ((rot >> t) & 1u) && r2r <= K.rc2;
-                const float r2 = SWITCH ? (on ? r2r : 1e30f) : r2r;   // as in the whole-entry kernel
-                const float rinv = rsqrt_ftz(r2);
-                const float r = r2 * rinv, rinv2 = rinv * rinv, rinv6 = rinv2 * rinv2 * rinv2;
-                const float4 ab = at_bytes(ljt, stl[t] + tj);      // A, B, 12A, 6B
-                float U = rinv6 * fmaf(ab.x, rinv6, -ab.y);
-                float G = (rinv6 * rinv2) * fmaf(ab.z, rinv6, -ab.w);
-                if (SWITCH) {
-                    const float x = __saturatef(fmaf(r, K.inv_sw, -K.rsw_inv)), x2 = x * x;
-                    const float S = fmaf(x2 * x, fmaf(x, fmaf(x, -6.f, 15.f), -10.f), 1.f);
-                    const float dSr = x2 * fmaf(x, fmaf(x, K.d30, K.d60), K.d30) * rinv;   // dS/dr / r
-                    G = fmaf(S, G, -U * dSr);
-                    U = U * S;
+        int p = b0;
+        do {
+            const int pe1 = PARTS ? min(p + part, b1) : b1;
+            double e_lj = 0, e_dir = 0;
+            float fix = 0, fiy = 0, fiz = 0;
+            for (int b = p; b < pe1; b += 4) {
+                const int e = b + eslot;
+                const PairEntry pe = pn;
+                if (e + 4 < b1) {
+                    pn = plist[L.start + e + 4];
                 } else {
-                    const float uc = ab.x * K.uc12 - ab.y * K.uc6;
-                    const float gc = (ab.z * K.uc12 - ab.w * K.uc6) / K.rc2f;
-                    U = U - uc + (r - K.rcf) * (gc * K.rcf);
-                    G = G - gc * K.rcf * rinv;
+                    pn.j = I; pn.shift = 13; pn.mask = 0ull;
                 }
-                const float ex = ex2_approx(K.kex * r2);
-                const float erfcv = erfc_as(rcp_ftz(fmaf(K.pa, r, 1.0f)), ex);
-                const float qq = xi.w * xj.w;
-                const float ec = qq * erfcv * rinv;
-                float g = fmaf(fmaf(qq * K.two_a_spi, ex, ec), rinv2, G);
-                if (!SWITCH) g = on ? g : 0.f;
+                const int J = pe.j;
+                const float4 xj = xq[J * CLUSTER + jj];
+                const int tj = stype[J * CLUSTER + jj] * (int)sizeof(float4);
+                const float4 cJ = centerf[J];
+                const float* s6 = sh[pe.shift];
+                // the j atom in I's frame: x_j - D, D = (c_I - c_J) - image offset
+                const float pjx = xj.x - (((cI.x - cJ.x) - s6[0]) - s6[3]);
+                const float pjy = xj.y - (((cI.y - cJ.y) - s6[1]) - s6[4]);
+                const float pjz = xj.z - (((cI.z - cJ.z) - s6[2]) - s6[5]);
+                // mask bits (4h + i) * 8 + jj, i = 0..3, rotated so step t tests bit t
+                const unsigned long long mc = pe.mask >> (32 * h + jj);
+                const unsigned nib = (unsigned)((mc & 1ull) | ((mc >> 7) & 2ull) | ((mc >> 14) & 4ull) | ((mc >> 21) & 8ull));
+                const unsigned rot = ((nib >> i4) | (nib << (4 - i4))) & 0xfu;
+                float fjx = 0.f, fjy = 0.f, fjz = 0.f, el = 0.f, ed = 0.f;
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const float4 xi = sxl[t];
+                    const float dx = xi.x - pjx, dy = xi.y - pjy, dz = xi.z - pjz;
+                    const float r2r = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                    const bool on = ((rot >> t) & 1u) && r2r <= K.rc2;
+                    const float r2 = SWITCH ? (on ? r2r : 1e30f) : r2r;   // as in the whole-entry kernel
+                    const float rinv = rsqrt_ftz(r2);
+                    const float r = r2 * rinv, rinv2 = rinv * rinv, rinv6 = rinv2 * rinv2 * rinv2;
+                    const float4 ab = at_bytes(ljt, stl[t] + tj);      // A, B, 12A, 6B
+                    float U = rinv6 * fmaf(ab.x, rinv6, -ab.y);
+                    float G = (rinv6 * rinv2) * fmaf(ab.z, rinv6, -ab.w);
+                    if (SWITCH) {
+                        const float x = __saturatef(fmaf(r, K.inv_sw, -K.rsw_inv)), x2 = x * x;
+                        const float S = fmaf(x2 * x, fmaf(x, fmaf(x, -6.f, 15.f), -10.f), 1.f);
+                        const float dSr = x2 * fmaf(x, fmaf(x, K.d30, K.d60), K.d30) * rinv;   // dS/dr / r
+                        G = fmaf(S, G, -U * dSr);
+                        U = U * S;
+                    } else {
+                        const float uc = ab.x * K.uc12 - ab.y * K.uc6;
+                        const float gc = (ab.z * K.uc12 - ab.w * K.uc6) / K.rc2f;
+                        U = U - uc + (r - K.rcf) * (gc * K.rcf);
+                        G = G - gc * K.rcf * rinv;
+                    }
+                    const float ex = ex2_approx(K.kex * r2);
+                    const float erfcv = erfc_as(rcp_ftz(fmaf(K.pa, r, 1.0f)), ex);
+                    const float qq = xi.w * xj.w;
+                    const float ec = qq * erfcv * rinv;
+                    float g = fmaf(fmaf(qq * K.two_a_spi, ex, ec), rinv2, G);
+                    if (!SWITCH) g = on ? g : 0.f;
+                    if (ENERGY) {
+                        el += SWITCH ? U : (on ? U : 0.f);
+                        ed += SWITCH ? ec : (on ? ec : 0.f);
+                    }
+                    if (COUNT) npc += on ? 1 : 0;
+                    fix = fmaf(g, dx, fix); fiy = fmaf(g, dy, fiy); fiz = fmaf(g, dz, fiz);
+                    fjx = fmaf(-g, dx, fjx); fjy = fmaf(-g, dy, fjy); fjz = fmaf(-g, dz, fjz);
+                    fix = __shfl_sync(FULL, fix, rot_src);
+                    fiy = __shfl_sync(FULL, fiy, rot_src);
+                    fiz = __shfl_sync(FULL, fiz, rot_src);
+                }
                 if (ENERGY) {
-                    el += SWITCH ? U : (on ? U : 0.f);
-                    ed += SWITCH ? ec : (on ? ec : 0.f);
+                    e_lj += (double)el;
+                    e_dir += (double)ed;
                 }
-                if (COUNT) npc += on ? 1 : 0;
-                fix = fmaf(g, dx, fix); fiy = fmaf(g, dy, fiy); fiz = fmaf(g, dz, fiz);
-                fjx = fmaf(-g, dx, fjx); fjy = fmaf(-g, dy, fjy); fjz = fmaf(-g, dz, fjz);
-                fix = __shfl_sync(FULL, fix, rot_src);
-                fiy = __shfl_sync(FULL, fiy, rot_src);
-                fiz = __shfl_sync(FULL, fiz, rot_src);
+                if (e < b1 && (fjx != 0.f || fjy != 0.f || fjz != 0.f)) {
+                    const int sl = J * CLUSTER + jj;
+                    fx_add_force_f(fslot + sl, fjx, st);
+                    fx_add_force_f(fslot + nslots + sl, fjy, st);
+                    fx_add_force_f(fslot + 2 * nslots + sl, fjz, st);
+                }
+            }
+            // lane jj holds a partial sum for i atom jj & 3: eight per atom
+#pragma unroll
+            for (int o = 4; o <= 16; o <<= 1) {
+                fix += __shfl_xor_sync(FULL, fix, o);
+                fiy += __shfl_xor_sync(FULL, fiy, o);
+                fiz += __shfl_xor_sync(FULL, fiz, o);
+            }
+            if (lane < 4) {
+                const int sl = I * CLUSTER + 4 * h + lane;
+                fx_add_force_f(fslot + sl, fix, st);
+                fx_add_force_f(fslot + nslots + sl, fiy, st);
+                fx_add_force_f(fslot + 2 * nslots + sl, fiz, st);
             }
             if (ENERGY) {
-                e_lj += (double)el;
-                e_dir += (double)ed;
+                const double s_lj = warp_sum(e_lj), s_dir = warp_sum(e_dir);
+                if (lane == 0) {
+                    if (s_lj != 0.0) fx_add(A.acc + MDF_E_VDW, s_lj, ENERGY_SCALE, st);
+                    if (s_dir != 0.0) fx_add(A.acc + MDF_E_EE_DIRECT, s_dir, ENERGY_SCALE, st);
+                }
             }
-            if (e < L.count && (fjx != 0.f || fjy != 0.f || fjz != 0.f)) {
-                const int sl = J * CLUSTER + jj;
-                fx_add_force_f(fslot + sl, fjx, st);
-                fx_add_force_f(fslot + nslots + sl, fjy, st);
-                fx_add_force_f(fslot + 2 * nslots + sl, fjz, st);
-            }
-        }
-        // lane jj holds a partial sum for i atom jj & 3: eight per atom
-        fix += __shfl_xor_sync(FULL, fix, 4); fix += __shfl_xor_sync(FULL, fix, 8); fix += __shfl_xor_sync(FULL, fix, 16);
-        fiy += __shfl_xor_sync(FULL, fiy, 4); fiy += __shfl_xor_sync(FULL, fiy, 8); fiy += __shfl_xor_sync(FULL, fiy, 16);
-        fiz += __shfl_xor_sync(FULL, fiz, 4); fiz += __shfl_xor_sync(FULL, fiz, 8); fiz += __shfl_xor_sync(FULL, fiz, 16);
-        if (lane < 4) {
-            const int sl = I * CLUSTER + 4 * h + lane;
-            fx_add_force_f(fslot + sl, fix, st);
-            fx_add_force_f(fslot + nslots + sl, fiy, st);
-            fx_add_force_f(fslot + 2 * nslots + sl, fiz, st);
-        }
-        if (ENERGY) {
-            const double s_lj = warp_sum(e_lj), s_dir = warp_sum(e_dir);
-            if (lane == 0) {
-                if (s_lj != 0.0) fx_add(A.acc + MDF_E_VDW, s_lj, ENERGY_SCALE, st);
-                if (s_dir != 0.0) fx_add(A.acc + MDF_E_EE_DIRECT, s_dir, ENERGY_SCALE, st);
-            }
-        }
+            p = pe1;
+        } while (PARTS && p < b1);
         __syncwarp();   // the next item overwrites this warp's i atoms
     }
     if (COUNT) {
@@ -640,95 +688,96 @@ __device__ __forceinline__ void pairs_f32_half_body_t(SmemF32H& S, const PairF32
 
 #define MDF_PF32_UNPACK(A)                                                                                       \
     A.nlist, A.ilist, A.plist, A.xq, A.stype, A.centerf, A.lj4, A.ntp, A.lj_smem, A.kc, A.K, A.shifts, A.fslot,      \
-        A.nslots, A.acc, A.npairs, A.next, A.persist, A.st
+        A.nslots, A.acc, A.npairs, A.next, A.persist, A.split, A.part, A.st
 
 // Every pair kernel holds two forms of its body: with the LJ table copied to
 // shared memory (lj_smem, when it fits) and read from global memory.  Either
 // way the table loads in the pair loop have a known address space (a generic
 // pointer chosen at run time measured 5% slower at 100k atoms).
-template <bool ENERGY, bool SWITCH, bool COUNT>
+template <bool ENERGY, bool SWITCH, bool COUNT, bool PARTS>
 __device__ __forceinline__ void pairs_f32_body(const PairF32Args& A)
 {
     __shared__ SmemF32W S;
-    if (A.lj_smem) pairs_f32_body_t<ENERGY, SWITCH, COUNT, true>(S, MDF_PF32_UNPACK(A));
-    else pairs_f32_body_t<ENERGY, SWITCH, COUNT, false>(S, MDF_PF32_UNPACK(A));
+    if (A.lj_smem) pairs_f32_body_t<ENERGY, SWITCH, COUNT, true, PARTS>(S, MDF_PF32_UNPACK(A));
+    else pairs_f32_body_t<ENERGY, SWITCH, COUNT, false, PARTS>(S, MDF_PF32_UNPACK(A));
 }
 
-template <bool ENERGY, bool SWITCH, bool COUNT>
+template <bool ENERGY, bool SWITCH, bool COUNT, bool PARTS>
 __device__ __forceinline__ void pairs_f32_half_body(const PairF32Args& A)
 {
     __shared__ SmemF32H S;
-    if (A.lj_smem) pairs_f32_half_body_t<ENERGY, SWITCH, COUNT, true>(S, A);
-    else pairs_f32_half_body_t<ENERGY, SWITCH, COUNT, false>(S, A);
+    if (A.lj_smem) pairs_f32_half_body_t<ENERGY, SWITCH, COUNT, true, PARTS>(S, A);
+    else pairs_f32_half_body_t<ENERGY, SWITCH, COUNT, false, PARTS>(S, A);
 }
 
 // With energies: up to 80 registers, three blocks per SM (left to itself the
 // compiler picks 64 and spills, which measured 1-2% slower).
-template <bool SWITCH, bool COUNT>
+template <bool SWITCH, bool COUNT, bool PARTS>
 __global__ void __launch_bounds__(NB_THREADS, 3) k_pairs_f32(PairF32Args A)
 {
-    pairs_f32_body<true, SWITCH, COUNT>(A);
+    pairs_f32_body<true, SWITCH, COUNT, PARTS>(A);
 }
 
 // Forces only (every dynamics step but the last of a chunk): 64 registers
 // with no spills, four blocks per SM (+4% dynamics steps/s).
-template <bool SWITCH, bool COUNT>
+template <bool SWITCH, bool COUNT, bool PARTS>
 __global__ void __launch_bounds__(NB_THREADS, 4) k_pairs_f32_force(PairF32Args A)
 {
-    pairs_f32_body<false, SWITCH, COUNT>(A);
+    pairs_f32_body<false, SWITCH, COUNT, PARTS>(A);
 }
 
 // The half-entry (4 x 8) forms, same register budgets.
-template <bool SWITCH, bool COUNT>
+template <bool SWITCH, bool COUNT, bool PARTS>
 __global__ void __launch_bounds__(NB_THREADS) k_pairs_f32_half(PairF32Args A)
 {
-    pairs_f32_half_body<true, SWITCH, COUNT>(A);
+    pairs_f32_half_body<true, SWITCH, COUNT, PARTS>(A);
 }
 
-template <bool SWITCH, bool COUNT>
+template <bool SWITCH, bool COUNT, bool PARTS>
 __global__ void __launch_bounds__(NB_THREADS, 4) k_pairs_f32_half_force(PairF32Args A)
 {
-    pairs_f32_half_body<false, SWITCH, COUNT>(A);
+    pairs_f32_half_body<false, SWITCH, COUNT, PARTS>(A);
 }
 
 // The many-system kernels hold one form of the body: LJS is the batch's
-// choice for all its systems (shared memory when every system's table fits).
-template <bool SWITCH, bool LJS>
+// choice for all its systems (shared memory when every system's table fits),
+// PARTS whether any system's lists are cut into parts.
+template <bool SWITCH, bool LJS, bool PARTS>
 __global__ void __launch_bounds__(NB_THREADS) k_pairs_f32_half_multi(const PairF32Args* __restrict__ As)
 {
     __shared__ SmemF32H S;
     const PairF32Args& A = As[blockIdx.z];
     if ((int)blockIdx.x >= A.gx) return;
-    pairs_f32_half_body_t<true, SWITCH, false, LJS>(S, A);
+    pairs_f32_half_body_t<true, SWITCH, false, LJS, PARTS>(S, A);
 }
 
-template <bool SWITCH, bool LJS>
+template <bool SWITCH, bool LJS, bool PARTS>
 __global__ void __launch_bounds__(NB_THREADS, 4) k_pairs_f32_half_force_multi(const PairF32Args* __restrict__ As)
 {
     __shared__ SmemF32H S;
     const PairF32Args& A = As[blockIdx.z];
     if ((int)blockIdx.x >= A.gx) return;
-    pairs_f32_half_body_t<false, SWITCH, false, LJS>(S, A);
+    pairs_f32_half_body_t<false, SWITCH, false, LJS, PARTS>(S, A);
 }
 
 // Many systems in one launch (blockIdx.z = system), with the same register
 // budgets as the one-system kernels above.
-template <bool SWITCH, bool LJS>
+template <bool SWITCH, bool LJS, bool PARTS>
 __global__ void __launch_bounds__(NB_THREADS, 3) k_pairs_f32_multi(const PairF32Args* __restrict__ As)
 {
     __shared__ SmemF32W S;
     const PairF32Args& A = As[blockIdx.z];
     if ((int)blockIdx.x >= A.gx) return;
-    pairs_f32_body_t<true, SWITCH, false, LJS>(S, MDF_PF32_UNPACK(A));
+    pairs_f32_body_t<true, SWITCH, false, LJS, PARTS>(S, MDF_PF32_UNPACK(A));
 }
 
-template <bool SWITCH, bool LJS>
+template <bool SWITCH, bool LJS, bool PARTS>
 __global__ void __launch_bounds__(NB_THREADS, 4) k_pairs_f32_force_multi(const PairF32Args* __restrict__ As)
 {
     __shared__ SmemF32W S;
     const PairF32Args& A = As[blockIdx.z];
     if ((int)blockIdx.x >= A.gx) return;
-    pairs_f32_body_t<false, SWITCH, false, LJS>(S, MDF_PF32_UNPACK(A));
+    pairs_f32_body_t<false, SWITCH, false, LJS, PARTS>(S, MDF_PF32_UNPACK(A));
 }
 #undef MDF_PF32_UNPACK
 
@@ -778,9 +827,9 @@ __device__ __forceinline__ void pairs_f64_body_t(SmemF64W& S, const PairF64Args&
             w = blockIdx.x * (blockDim.x >> 5) + wib;
         }
         if (w >= nlist) break;
-        double e_lj = 0, e_dir = 0;
-        double fix = 0, fiy = 0, fiz = 0;
         const ILRange L = ilist[w];
+        const int b1 = L.count;
+        if (b1 == 0) continue;
         const int I = L.i;
         const double4 xi = xq[I * CLUSTER + ii];
         const int trow = stype[I * CLUSTER + ii] * ntp * (int)sizeof(double4);   // byte offsets
@@ -790,15 +839,17 @@ __device__ __forceinline__ void pairs_f64_body_t(SmemF64W& S, const PairF64Args&
         const int rot_src = (lane & ~7) | ((ii + 1) & 7);
         // the lane's entry of the next batch is loaded one batch ahead
         PairEntry pn;
-        if (jslot < L.count) {
+        if (jslot < b1) {
             pn = plist[L.start + jslot];
         } else {
             pn.j = I; pn.shift = 13; pn.mask = 0ull;
         }
-        for (int b = 0; b < L.count; b += 4) {
+        double e_lj = 0, e_dir = 0;
+        double fix = 0, fiy = 0, fiz = 0;
+        for (int b = 0; b < b1; b += 4) {
             const int e = b + jslot;
             const PairEntry pe = pn;
-            if (e + 4 < L.count) {
+            if (e + 4 < b1) {
                 pn = plist[L.start + e + 4];
             } else {
                 pn.j = I; pn.shift = 13; pn.mask = 0ull;
@@ -861,10 +912,10 @@ __device__ __forceinline__ void pairs_f64_body_t(SmemF64W& S, const PairF64Args&
                 fjz = __shfl_sync(FULL, fjz, rot_src);
             }
             if (ENERGY) {
-                e_lj += el;
-                e_dir += ed;
+                e_lj += (double)el;
+                e_dir += (double)ed;
             }
-            if (e < L.count && (fjx != 0.0 || fjy != 0.0 || fjz != 0.0)) {
+            if (e < b1 && (fjx != 0.0 || fjy != 0.0 || fjz != 0.0)) {
                 const int sl = J * CLUSTER + ii;
                 fx_add(fslot + sl, fjx, FORCE_SCALE, st);
                 fx_add(fslot + nslots + sl, fjy, FORCE_SCALE, st);
@@ -934,6 +985,8 @@ __device__ __forceinline__ void pairs_f64_half_body_t(SmemF64H& S, const PairF64
         }
         if (w >= nlist) break;
         const ILRange L = ilist[w];
+        const int b1 = L.count;
+        if (b1 == 0) continue;
         const int I = L.i, h = L.pad;
         if (lane < 8) {
             double4 v = xq[I * CLUSTER + 4 * h + (lane & 3)];
@@ -945,19 +998,19 @@ __device__ __forceinline__ void pairs_f64_half_body_t(SmemF64H& S, const PairF64
         const double4 cI = center[I];
         const double4* __restrict__ sxl = &sxi[wib][i4];
         const int* __restrict__ stl = &sti[wib][i4];
-        double e_lj = 0, e_dir = 0;
-        double fix = 0, fiy = 0, fiz = 0;
         // the lane's entry of the next batch is loaded one batch ahead
         PairEntry pn;
-        if (eslot < L.count) {
+        if (eslot < b1) {
             pn = plist[L.start + eslot];
         } else {
             pn.j = I; pn.shift = 13; pn.mask = 0ull;
         }
-        for (int b = 0; b < L.count; b += 4) {
+        double e_lj = 0, e_dir = 0;
+        double fix = 0, fiy = 0, fiz = 0;
+        for (int b = 0; b < b1; b += 4) {
             const int e = b + eslot;
             const PairEntry pe = pn;
-            if (e + 4 < L.count) {
+            if (e + 4 < b1) {
                 pn = plist[L.start + e + 4];
             } else {
                 pn.j = I; pn.shift = 13; pn.mask = 0ull;
@@ -1015,19 +1068,22 @@ __device__ __forceinline__ void pairs_f64_half_body_t(SmemF64H& S, const PairF64
                 fiz = __shfl_sync(FULL, fiz, rot_src);
             }
             if (ENERGY) {
-                e_lj += el;
-                e_dir += ed;
+                e_lj += (double)el;
+                e_dir += (double)ed;
             }
-            if (e < L.count && (fjx != 0.0 || fjy != 0.0 || fjz != 0.0)) {
+            if (e < b1 && (fjx != 0.0 || fjy != 0.0 || fjz != 0.0)) {
                 const int sl = J * CLUSTER + jj;
                 fx_add(fslot + sl, fjx, FORCE_SCALE, st);
                 fx_add(fslot + nslots + sl, fjy, FORCE_SCALE, st);
                 fx_add(fslot + 2 * nslots + sl, fjz, FORCE_SCALE, st);
             }
         }
-        fix += __shfl_xor_sync(FULL, fix, 4); fix += __shfl_xor_sync(FULL, fix, 8); fix += __shfl_xor_sync(FULL, fix, 16);
-        fiy += __shfl_xor_sync(FULL, fiy, 4); fiy += __shfl_xor_sync(FULL, fiy, 8); fiy += __shfl_xor_sync(FULL, fiy, 16);
-        fiz += __shfl_xor_sync(FULL, fiz, 4); fiz += __shfl_xor_sync(FULL, fiz, 8); fiz += __shfl_xor_sync(FULL, fiz, 16);
+#pragma unroll
+        for (int o = 4; o <= 16; o <<= 1) {
+            fix += __shfl_xor_sync(FULL, fix, o);
+            fiy += __shfl_xor_sync(FULL, fiy, o);
+            fiz += __shfl_xor_sync(FULL, fiz, o);
+        }
         if (lane < 4) {
             const int sl = I * CLUSTER + 4 * h + lane;
             fx_add(fslot + sl, fix, FORCE_SCALE, st);
@@ -1288,6 +1344,26 @@ NBParams make_params(const Ctx& c)
     return P;
 }
 
+// Entries per part: a property of the system (not of a rank's share or of the
+// batch it is in), since it sets the order of the sums.  The extra reductions
+// cost the pair kernel about 3% and above SPLIT_CLUSTERS buy nothing.  FP32
+// only: the parts' fixed-point rounding (2^-32 each) lies far below FP32
+// sums, but would show in the last digits of the FP64 ones.
+static int pair_part(const Ctx& c)
+{
+    return c.n_clusters < SPLIT_CLUSTERS ? PART_ENTRIES : WHOLE_LIST;
+}
+
+// log2 of the shares each of nlist lists is cut into: enough items for one
+// wave of three 8-warp blocks per SM (148 * 24 = 3552).  At 372 lists 22 us
+// with eight shares, 25 with four, 35 with two.
+int pair_split(long long nlist)
+{
+    int s = 0;
+    while (s < 3 && (nlist << s) < 3552) ++s;
+    return s;
+}
+
 // Warps per block of the pair kernels: mdf_params.pair_warps (2, 4 or 8; 0 = 8).
 static int pair_warps(const Ctx& c)
 {
@@ -1436,16 +1512,12 @@ PairF32Args make_pair_f32_args(const Ctx& c, size_t* dyn)
     long long lo, hi;
     cluster_share(c, lo, hi);   // this rank's i clusters
     A.nlist = (int)(hi - lo);
-    A.gx = grid_blocks(A.nlist, wpb);
     A.gy = 1;
     const bool pruned = c.p.prune_every != 0 && c.pruned_valid;
     A.half = pruned && c.pruned_half ? 1 : 0;
     A.ilist = A.half ? c.ilist_h.p + 2 * lo : (pruned ? c.ilist_in.p : c.ilist.p) + lo;
     A.plist = pruned ? (A.half ? c.plist_h.p : c.plist_in.p) : c.plist.p;
-    if (A.half) {
-        A.nlist *= 2;   // two half items per i cluster
-        A.gx = grid_blocks(A.nlist, wpb);
-    }
+    if (A.half) A.nlist *= 2;   // two half lists per i cluster
     A.xq = c.xq_f.p;
     A.stype = c.slot_type.p;
     A.centerf = c.centerf.p;
@@ -1459,6 +1531,8 @@ PairF32Args make_pair_f32_args(const Ctx& c, size_t* dyn)
     A.next = c.scal.p + SCAL_WORK;
     A.persist = c.p.pair_schedule == 1 ? 1 : 0;
     A.st = c.status.p;
+    A.part = pair_part(c);
+    set_pair_split(A, pair_split(A.nlist), wpb);
     return A;
 }
 
@@ -1470,22 +1544,28 @@ static void launch_pairs_f32(Ctx& c, bool energy)
     if (A.nlist == 0) return;
     const int th = 32 * pair_warps(c);
     const bool sw = c.p.switch_radius > 0.0;
-#define MDF_PF32(E, S, K_)                                                                                     \
+#define MDF_PF32(E, S, K_, P_)                                                                                     \
     do {                                                                                                       \
-        const void* fn = A.half ? ((E) ? (const void*)k_pairs_f32_half<S, K_>                                  \
-                                       : (const void*)k_pairs_f32_half_force<S, K_>)                           \
-                                : ((E) ? (const void*)k_pairs_f32<S, K_> : (const void*)k_pairs_f32_force<S, K_>); \
+        const void* fn = A.half ? ((E) ? (const void*)k_pairs_f32_half<S, K_, P_>                                  \
+                                       : (const void*)k_pairs_f32_half_force<S, K_, P_>)                           \
+                                : ((E) ? (const void*)k_pairs_f32<S, K_, P_> : (const void*)k_pairs_f32_force<S, K_, P_>); \
         const int nb = A.persist ? std::min(A.gx, persistent_blocks(fn, th, dyn)) : A.gx;                       \
         if (A.half) {                                                                                          \
-            if (E) k_pairs_f32_half<S, K_><<<nb, th, dyn, c.stream>>>(A);                                        \
-            else k_pairs_f32_half_force<S, K_><<<nb, th, dyn, c.stream>>>(A);                                    \
+            if (E) k_pairs_f32_half<S, K_, P_><<<nb, th, dyn, c.stream>>>(A);                                        \
+            else k_pairs_f32_half_force<S, K_, P_><<<nb, th, dyn, c.stream>>>(A);                                    \
         } else {                                                                                               \
-            if (E) k_pairs_f32<S, K_><<<nb, th, dyn, c.stream>>>(A);                                             \
-            else k_pairs_f32_force<S, K_><<<nb, th, dyn, c.stream>>>(A);                                         \
+            if (E) k_pairs_f32<S, K_, P_><<<nb, th, dyn, c.stream>>>(A);                                             \
+            else k_pairs_f32_force<S, K_, P_><<<nb, th, dyn, c.stream>>>(A);                                         \
         }                                                                                                      \
     } while (0)
 #define MDF_PF32_K(E, S) \
-    do { if (count) MDF_PF32(E, S, true); else MDF_PF32(E, S, false); } while (0)
+    do {                                                                                                       \
+        if (A.part < WHOLE_LIST) {                                                                             \
+            if (count) MDF_PF32(E, S, true, true); else MDF_PF32(E, S, false, true);                             \
+        } else {                                                                                               \
+            if (count) MDF_PF32(E, S, true, false); else MDF_PF32(E, S, false, false);                           \
+        }                                                                                                      \
+    } while (0)
     if (energy) {
         if (sw) MDF_PF32_K(true, true); else MDF_PF32_K(true, false);
     } else {
@@ -1498,29 +1578,32 @@ static void launch_pairs_f32(Ctx& c, bool energy)
 }
 
 void launch_pairs_f32_multi(const PairF32Args* d_args, int nsys, int gx, int threads, size_t dyn, bool energy,
-                            bool use_switch, bool persist, bool half, bool lj_smem, cudaStream_t s)
+                            bool use_switch, bool persist, bool half, bool lj_smem, bool parts, cudaStream_t s)
 {
 #define MDF_PF32M(KERN)                                                                                        \
     do {                                                                                                       \
         const dim3 g(persist ? std::min(gx, persistent_blocks((const void*)KERN, threads, dyn)) : gx, 1, nsys); \
         KERN<<<g, threads, dyn, s>>>(d_args);                                                                  \
     } while (0)
-#define MDF_PF32S(S, L)                                                                                        \
+#define MDF_PF32P(S, L, P_)                                                                                       \
     do {                                                                                                       \
         if (half) {                                                                                            \
-            if (energy) MDF_PF32M((k_pairs_f32_half_multi<S, L>));                                             \
-            else MDF_PF32M((k_pairs_f32_half_force_multi<S, L>));                                              \
+            if (energy) MDF_PF32M((k_pairs_f32_half_multi<S, L, P_>));                                             \
+            else MDF_PF32M((k_pairs_f32_half_force_multi<S, L, P_>));                                              \
         } else {                                                                                               \
-            if (energy) MDF_PF32M((k_pairs_f32_multi<S, L>));                                                  \
-            else MDF_PF32M((k_pairs_f32_force_multi<S, L>));                                                   \
+            if (energy) MDF_PF32M((k_pairs_f32_multi<S, L, P_>));                                                  \
+            else MDF_PF32M((k_pairs_f32_force_multi<S, L, P_>));                                                   \
         }                                                                                                      \
     } while (0)
+#define MDF_PF32S(S, L) \
+    do { if (parts) MDF_PF32P(S, L, true); else MDF_PF32P(S, L, false); } while (0)
     if (use_switch) {
         if (lj_smem) MDF_PF32S(true, true); else MDF_PF32S(true, false);
     } else {
         if (lj_smem) MDF_PF32S(false, true); else MDF_PF32S(false, false);
     }
 #undef MDF_PF32S
+#undef MDF_PF32P
 #undef MDF_PF32M
     MDF_CUDA_TRY(cudaGetLastError());
 }
@@ -1553,16 +1636,12 @@ PairF64Args make_pair_f64_args(const Ctx& c, size_t* dyn)
     long long lo, hi;
     cluster_share(c, lo, hi);   // this rank's i clusters
     A.nlist = (int)(hi - lo);
-    A.gx = grid_blocks(A.nlist, wpb);
     A.gy = 1;
     const bool pruned = c.p.prune_every != 0 && c.pruned_valid;
     A.half = pruned && c.pruned_half ? 1 : 0;
     A.ilist = A.half ? c.ilist_h.p + 2 * lo : (pruned ? c.ilist_in.p : c.ilist.p) + lo;
     A.plist = pruned ? (A.half ? c.plist_h.p : c.plist_in.p) : c.plist.p;
-    if (A.half) {
-        A.nlist *= 2;   // two half items per i cluster
-        A.gx = grid_blocks(A.nlist, wpb);
-    }
+    if (A.half) A.nlist *= 2;   // two half lists per i cluster
     A.xq = c.xq_d.p;
     A.stype = c.slot_type.p;
     A.center = c.center.p;
@@ -1576,6 +1655,7 @@ PairF64Args make_pair_f64_args(const Ctx& c, size_t* dyn)
     A.next = c.scal.p + SCAL_WORK;
     A.persist = c.p.pair_schedule == 1 ? 1 : 0;
     A.st = c.status.p;
+    A.gx = grid_blocks(A.nlist, wpb);
     return A;
 }
 
