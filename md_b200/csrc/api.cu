@@ -790,7 +790,7 @@ void mdf_destroy(mdf_ctx* ctx)
     c.col_atoms.release(); c.slot_atom.release(); c.atom_slot.release(); c.slot_type.release(); c.center.release(); c.centerf.release();
     c.bb_lo.release(); c.bb_hi.release(); c.xq_f.release(); c.xq_d.release(); c.cluster_col.release();
     c.ilist.release(); c.plist.release(); c.scan_tmp.release(); c.f_slot.release();
-    c.plist_in.release(); c.ilist_in.release(); c.cur_lo.release(); c.cur_hi.release(); c.xq_snap.release();
+    c.plist_in.release(); c.ilist_in.release(); c.cur_box.release(); c.xq_snap.release();
     c.q_slab.release(); c.pme_slab.release(); c.pme_send.release(); c.pme_recv.release(); c.pme_rslab.release();
     c.f_stage.release(); c.f_mine.release(); c.f_out_blk.release(); c.f_out_all.release();
     c.f_atom.release(); c.scal.release(); c.npairs_dev.release(); c.forces_out.release(); c.forces_pme_ref.release();

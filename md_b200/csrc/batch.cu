@@ -190,7 +190,7 @@ bool uniform_launches(const mdf_batch* b)
 template <typename R>
 struct MultiArgs {
     std::vector<PackArgs<R>> pack;
-    std::vector<PruneArgs<R>> prune;
+    std::vector<PruneArgs> prune;
     std::vector<PairF32Args> pf32;
     std::vector<PairF64Args> p64;
     std::vector<ExclArgs> excl;
@@ -211,6 +211,7 @@ struct MultiArgs {
     size_t dyn_pairs = 0;
     int threads = 256;
     bool prune_on = false, use_switch = false, energy = false, persist = false, half = false;
+    int prune_warps = 1;
     bool parts = false;    // some system's lists are cut into parts
     bool lj_smem = true;   // every system's LJ table in shared memory (one kernel form for the batch)
 };
@@ -218,7 +219,7 @@ struct MultiArgs {
 template <typename R>
 struct MultiDev {
     const PackArgs<R>* pack;
-    const PruneArgs<R>* prune;
+    const PruneArgs* prune;
     const PairF32Args* pf32;
     const PairF64Args* p64;
     const ExclArgs* excl;
@@ -280,7 +281,7 @@ MultiDev<R> prepare_multi(mdf_batch* b, uint32_t flags, MultiArgs<R>& M, double*
             c.pruned_half = M.half;
         }
         M.pack.push_back(make_pack_args<R>(c));
-        M.prune.push_back(M.half ? make_prune_half_args<R>(c) : make_prune_args<R>(c));
+        M.prune.push_back(make_prune_args(c, M.half));
         if (sizeof(R) == 4) {
             size_t dyn = 0;
             M.pf32.push_back(make_pair_f32_args(c, &dyn));
@@ -331,8 +332,11 @@ MultiDev<R> prepare_multi(mdf_batch* b, uint32_t flags, MultiArgs<R>& M, double*
         for (auto& a : M.p64) a.lj_smem = 0;
         M.dyn_pairs = 0;
     }
-    // shares of the pair lists: by the work of the whole batch
-    long long nlist = 0;
+    // warps per cluster of the prune and shares of the pair lists: by the work of the whole batch
+    long long ncl = 0, nlist = 0;
+    for (const auto& a : M.prune) ncl += a.ncl;
+    for (auto& a : M.prune) set_prune_warps(a, ncl);
+    M.prune_warps = M.prune[0].warps;
     for (const auto& a : M.pf32) nlist += a.nlist;
     for (auto& a : M.pf32) {
         set_pair_split(a, pair_split(nlist), M.threads / 32);
@@ -434,7 +438,7 @@ void enqueue_multi(mdf_batch* b, const MultiArgs<R>& M, const MultiDev<R>& D, co
     launch_pack_multi<R>(D.pack, D.pack_m, b->main);
     ++k;
     if (M.prune_on) {
-        launch_prune_multi<R>(D.prune, n, M.gx_prune, M.half, b->main);
+        launch_prune_multi(D.prune, n, M.gx_prune, M.prune_warps, M.half, self_pruning(b->sys[0]->c), b->main);
         ++k;
     }
     if (M.gx_pairs > 0) {

@@ -38,32 +38,33 @@ struct PackArgs {
     const double4* center;
     double L[3];
     typename V4<R>::type* xq;
-    float4 *cur_lo, *cur_hi;
+    float4* box;                        // current boxes (box_encode)
+    float box_pad;
+    float4* xf;                         // FP64: the FP32 copy of xq
     const typename V4<R>::type* snap;   // self-pruning: positions of the last prune (nullptr: off)
     unsigned* disp;                     // largest squared displacement from snap (FP32 bits, atomicMax)
     unsigned* st;
 };
 
-struct PruneShifts {
-    float v[27][6];
-};
-
-template <typename R>
 struct PruneArgs {
     int gx, gy;
     int ncl;
+    int warps;              // warps per i cluster: 1 or 4
     const ILRange* ilist;
     const PairEntry* plist;
-    const typename V4<R>::type* xq;
-    const float4 *centerf, *cur_lo, *cur_hi;
-    PruneShifts shifts;
+    const float4* xf;
+    const double4* xd;      // FP64 offsets (snap_d only)
+    const float4 *centerf, *box;
+    int box_fine;           // box padding small enough for the acceptance by boxes
+    ShiftTable shifts;
     float rcut2;
     ILRange* ilist_in;
     PairEntry* plist_in;
     // self-pruning: prune only when force is set or the displacement since the
     // last prune (written by the pack kernel) exceeds disp_thr2; a prune that
-    // runs records the positions it used in snap
-    typename V4<R>::type* snap;
+    // runs records the positions it used in the snapshot of the precision
+    float4* snap_f;
+    double4* snap_d;
     const unsigned* disp;
     float disp_thr2;
     int force;
@@ -352,11 +353,10 @@ struct FinalizeArgs {
 // many-system launchers (device arrays of arguments, the largest grid).
 template <typename R> PackArgs<R> make_pack_args(const Ctx& c);
 template <typename R> void launch_pack_multi(const PackArgs<R>* d_args, BlockMap bm, cudaStream_t s);
-template <typename R> PruneArgs<R> make_prune_args(const Ctx& c);
-template <typename R> PruneArgs<R> make_prune_half_args(const Ctx& c);
+PruneArgs make_prune_args(const Ctx& c, bool half);
+void set_prune_warps(PruneArgs& A, long long ncl);   // by the clusters of the whole launch
 void ensure_half_lists(Ctx& c);
-template <typename R>
-void launch_prune_multi(const PruneArgs<R>* d_args, int nsys, int gx, bool half, cudaStream_t s);
+void launch_prune_multi(const PruneArgs* d_args, int nsys, int gx, int warps, bool half, bool selfp, cudaStream_t s);
 PairF32Args make_pair_f32_args(const Ctx& c, size_t* dyn);
 void launch_pairs_f32_multi(const PairF32Args* d_args, int nsys, int gx, int threads, size_t dyn, bool energy,
                             bool use_switch, bool persist, bool half, bool lj_smem, bool parts, cudaStream_t s);

@@ -173,8 +173,8 @@ struct Ctx {
     DevBuf<float4> centerf;        // the same centres, exact in FP32 (they lie on a 2^-k grid)
     double center_quantum = 0.0;
     DevBuf<float4> bb_lo, bb_hi;   // [n_clusters] bounding boxes (wrapped coordinates)
-    DevBuf<float4> cur_lo, cur_hi; // [n_clusters] current boxes in the cluster frame (per evaluation)
-    DevBuf<float4> xq_f;           // [n_slots] offset from center + q (mixed)
+    DevBuf<float4> cur_box;        // [n_clusters] current boxes (per evaluation; box_encode)
+    DevBuf<float4> xq_f;           // [n_slots] offset from center + q (FP64 contexts: the prune's copy)
     DevBuf<double4> xq_d;          // [n_slots] (FP64)
     DevBuf<int> cluster_col;       // [n_clusters]
     DevBuf<ILRange> ilist;         // [n_clusters]

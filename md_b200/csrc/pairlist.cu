@@ -215,11 +215,45 @@ __global__ void k_cluster_geom(const int* __restrict__ d_ncl, const double* __re
     bb_hi[c] = make_float4(__double2float_ru(hi[0]), __double2float_ru(hi[1]), __double2float_ru(hi[2]), 0.f);
 }
 
+struct BoxF {
+    float x, y, z, hx, hy, hz;
+    bool fine;   // half extents to 1/64 A
+};
+
+// Box of a cluster in absolute coordinates: centre, and half extents in units
+// of 2^(4s-6) A, rounded up, as 3 x 10 bits with s in the top two.
+__device__ __forceinline__ float4 box_encode(const float lo[3], const float hi[3], const double4& c, float pad)
+{
+    float h[3], m = 0.f;
+    for (int k = 0; k < 3; ++k) {
+        h[k] = fmaxf(0.f, 0.5f * (hi[k] - lo[k])) + pad;   // + rounding of the centre
+        m = fmaxf(m, h[k]);
+    }
+    unsigned s = 0;
+    while (s < 3 && m > 1020.f * __uint_as_float((121u + 4u * s) << 23)) ++s;
+    const float per = __uint_as_float((133u - 4u * s) << 23);   // 2^(6-4s)
+    unsigned u = s << 30;
+    for (int k = 0; k < 3; ++k) u |= min(1023u, (unsigned)ceilf(h[k] * per)) << (10 * k);
+    const bool real = lo[0] <= hi[0];
+    return make_float4((float)c.x + (real ? 0.5f * (lo[0] + hi[0]) : 0.f),
+                       (float)c.y + (real ? 0.5f * (lo[1] + hi[1]) : 0.f),
+                       (float)c.z + (real ? 0.5f * (lo[2] + hi[2]) : 0.f), __uint_as_float(u));
+}
+
+__device__ __forceinline__ BoxF box_decode(const float4& b)
+{
+    const unsigned u = __float_as_uint(b.w);
+    const float unit = __uint_as_float((121u + 4u * (u >> 30)) << 23);
+    return BoxF{b.x, b.y, b.z, (float)(u & 1023u) * unit, (float)((u >> 10) & 1023u) * unit,
+                (float)((u >> 20) & 1023u) * unit, (u >> 30) == 0u};
+}
+
 // Per-evaluation packing: cluster-ordered offsets from the cluster centre
 // (min image, so atoms crossing the box edge between rebuilds stay whole)
 // plus charge, in the working precision.
-// Also the cluster's current bounding box in its own frame (FP32, rounded
-// outward) for the prune's box test.  blockDim.x must be a multiple of 32.
+// Also the cluster's current bounding box for the prune's box test
+// (box_encode) and, in FP64, the FP32 copy of the offsets that the prune reads.
+// blockDim.x must be a multiple of 32.
 template <typename R>
 __device__ __forceinline__ void pack_dev(const PackArgs<R>& A, int bx, int by)
 {
@@ -230,8 +264,6 @@ __device__ __forceinline__ void pack_dev(const PackArgs<R>& A, int bx, int by)
     const double4* __restrict__ center = A.center;
     const double Lx = A.L[0], Ly = A.L[1], Lz = A.L[2];
     typename V4<R>::type* __restrict__ xq = A.xq;
-    float4* __restrict__ cur_lo = A.cur_lo;
-    float4* __restrict__ cur_hi = A.cur_hi;
     unsigned* st = A.st;
     const int s = bx * blockDim.x + threadIdx.x;
     const bool inside = s < nslots;
@@ -255,6 +287,7 @@ __device__ __forceinline__ void pack_dev(const PackArgs<R>& A, int bx, int by)
         }
     }
     if (inside) xq[s] = v;
+    if (sizeof(R) == 8 && inside) A.xf[s] = make_float4((float)v.x, (float)v.y, (float)v.z, (float)v.w);
     if (A.snap) {
         // self-pruning: the largest squared displacement since the last prune
         float d2 = 0.f;
@@ -275,10 +308,7 @@ __device__ __forceinline__ void pack_dev(const PackArgs<R>& A, int bx, int by)
             lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
             hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
         }
-    if (inside && (s % CLUSTER) == 0) {
-        cur_lo[s / CLUSTER] = make_float4(lo[0], lo[1], lo[2], 0.f);
-        cur_hi[s / CLUSTER] = make_float4(hi[0], hi[1], hi[2], 0.f);
-    }
+    if (inside && (s % CLUSTER) == 0) A.box[s / CLUSTER] = box_encode(lo, hi, center[s / CLUSTER], A.box_pad);
 }
 
 template <typename R>
@@ -483,299 +513,251 @@ __global__ void k_exclusion_masks(int nexcl, const int* __restrict__ excl, const
 }
 
 // ------------------------------------------------------------- pruning
-// Two levels, one lane per outer entry.  Level 1 rejects the entry when the
-// current bounding boxes of the two clusters (k_pack) are rcut apart.  Level 2
-// loads the entry's eight j atoms (independent loads, all in flight at once),
-// skips every j atom farther than rcut from the i cluster's box, and tests the
-// rest against the eight i atoms (held in registers by every lane), stopping
-// at the first unmasked pair inside rcut.  Kept entries are compacted, in
-// list order, into the same offsets of the pruned list.  Image offsets use the
-// exact-FP32 centres plus the hi/lo shift table.
 // Dynamic pruning: keep the outer-list entries that have at least one atom
-// pair within the prune radius at the current positions.  Warp per i cluster.
-// The warp loads 32 entries at once (one per lane), drops those whose current
-// cluster boxes are farther apart than the radius, and checks the remaining
-// candidates four at a time with lane = (candidate, j atom): each lane tests
-// its j atom against the eight i atoms held in registers, and one ballot gives
-// the four keep flags.  The test ignores the entry's exclusion mask (an entry
-// whose only close pairs are excluded is kept; the pair kernel applies the
-// mask), so it keeps a superset of the exact set.  Distances use
-// |a - b|^2 = |a|^2 + |b|^2 - 2 a.b: three FMAs and a min per pair, the
-// rounding (~1e-4 A^2 at these magnitudes) far inside the radius' margin.
-// Kept entries are written in order, packed from the i cluster's start offset
-// in the outer list.
-template <typename R>
-__device__ __forceinline__ void prune_dev(const PruneArgs<R>& A)
+// pair within the prune radius at the current positions, in list order, packed
+// from the i cluster's start offset in the outer list.  The test ignores the
+// entry's exclusion mask (an entry whose only close pairs are excluded is
+// kept; the pair kernel applies the mask), so it keeps a superset of the exact
+// set, and it runs in FP32 in both precisions: the frame offsets are exact to
+// ~1e-6 A and |a - b|^2 = |a|^2 + |b|^2 - 2 a.b rounds by ~1e-4 A^2, far
+// inside the radius' 0.02 A margin.
+//
+// W warps share an i cluster (32 entries each per round).  An entry is first
+// tested lane by lane through the clusters' current boxes (k_pack): farther
+// apart than the radius - dropped; so close that two face atoms must lie
+// within it - kept.  The others go to shared memory and are tested eight at a
+// time, four lanes each with two j atoms against the eight i atoms in
+// registers as packed FP32x2 pairs (three FMAs per two pairs, one three-input
+// minimum).
+//
+// What bounds it: gathers and latency (half the issue slots used, 470 warp
+// instructions per 32 entries).  One lane per entry with early exit, the form
+// before, read 32 lines per load instruction and three 16-byte box words per
+// entry; here a box is one 16-byte word and a test reads eight whole lines.
+// FP32 at 100k atoms 48 -> 44 us, at 960k 408 -> 359 us; FP64 half lists at
+// 100k (FP64 arithmetic before) 125 -> 50 us.  Loading the next 32 entries and
+// boxes a round ahead gained nothing (42-52 us); at three blocks per SM,
+// without the 48 spilled bytes, 100k took 42 us but 960k 396 us.
+using F32x2 = unsigned long long;   // two packed FP32 values
+__device__ __forceinline__ F32x2 pack2(float lo, float hi)
 {
-    const int ncl = A.ncl;
-    const ILRange* __restrict__ ilist = A.ilist;
-    const PairEntry* __restrict__ plist = A.plist;
-    const typename V4<R>::type* __restrict__ xq = A.xq;
-    const float4* __restrict__ centerf = A.centerf;
-    const float4* __restrict__ cur_lo = A.cur_lo;
-    const float4* __restrict__ cur_hi = A.cur_hi;
-    const PruneShifts& shifts = A.shifts;
-    const float rcut2 = A.rcut2;
-    ILRange* __restrict__ ilist_in = A.ilist_in;
-    PairEntry* __restrict__ plist_in = A.plist_in;
-    using V4t = typename V4<R>::type;
+    F32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ F32x2 fma2(F32x2 a, F32x2 b, F32x2 c)
+{
+    F32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float min_with2(float m, F32x2 v)   // min(m, v.lo, v.hi)
+{
+    float lo, hi, r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(lo), "f"(hi));
+    return r;
+}
+
+constexpr int PRUNE_WARPS = 8;   // largest block
+
+// HALF: the half layout (4 x 8).  Each half of the i cluster (atoms 0-3, 4-7)
+// is tested on its own and an entry goes to the list of every half that has an
+// atom pair within the radius.  The outer range [start, start + count) of i
+// cluster I owns the slots [2 start + h count, 2 start + (h + 1) count) of the
+// half list; item 2 w + h of this launch describes half h (ILRange.pad = h).
+template <int W, bool HALF>
+__device__ __forceinline__ void prune_dev(const PruneArgs& A)
+{
     // self-pruning: the list pruned last time still holds every pair within the cutoff
     if (!A.force && __uint_as_float(*A.disp) <= A.disp_thr2) return;
     __shared__ float sh[27][6];
-    for (int k = threadIdx.x; k < 27 * 6; k += blockDim.x) sh[k / 6][k % 6] = shifts.v[k / 6][k % 6];
-    __syncthreads();
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;   // index into this launch's ilist range
-    const int lane = threadIdx.x & 31;
-    if (w >= ncl) return;
-    const unsigned below = (1u << lane) - 1u;
-    const ILRange L = ilist[w];
-    const int I = L.i;
-    if (A.snap && lane < CLUSTER) A.snap[I * CLUSTER + lane] = xq[I * CLUSTER + lane];
-    R ax[CLUSTER], ay[CLUSTER], az[CLUSTER], an[CLUSTER];   // -2 x_i and |x_i|^2
-#pragma unroll
-    for (int k = 0; k < CLUSTER; ++k) {
-        const V4t v = xq[I * CLUSTER + k];
-        ax[k] = (R)-2 * v.x; ay[k] = (R)-2 * v.y; az[k] = (R)-2 * v.z;
-        an[k] = v.x * v.x + v.y * v.y + v.z * v.z;
-    }
-    const float4 cI = centerf[I], ilo = cur_lo[I], ihi = cur_hi[I];
-    const R rc2 = (R)rcut2;
-    int kept = 0;
-    for (int base = 0; base < L.count; base += 32) {
-        const bool have = base + lane < L.count;
-        PairEntry my;
-        my.j = I; my.shift = 13; my.mask = 0ull;
-        if (have) my = plist[L.start + base + lane];
-        // this lane's entry: J's frame origin seen from I's frame, and the box test
-        const float4 cJ = centerf[my.j], jlo = cur_lo[my.j], jhi = cur_hi[my.j];
-        const float* s6 = sh[my.shift];
-        const float ox = -(((cI.x - cJ.x) - s6[0]) - s6[3]);
-        const float oy = -(((cI.y - cJ.y) - s6[1]) - s6[4]);
-        const float oz = -(((cI.z - cJ.z) - s6[2]) - s6[5]);
-        const float gx = fmaxf(0.f, fmaxf(jlo.x + ox - ihi.x, ilo.x - (jhi.x + ox)));
-        const float gy = fmaxf(0.f, fmaxf(jlo.y + oy - ihi.y, ilo.y - (jhi.y + oy)));
-        const float gz = fmaxf(0.f, fmaxf(jlo.z + oz - ihi.z, ilo.z - (jhi.z + oz)));
-        const bool cand = have && my.mask != 0ull && gx * gx + gy * gy + gz * gz < rcut2;
-        unsigned keepmask;
-        if constexpr (sizeof(R) == 4) {
-            // FP32: this lane's entry against all 64 atom pairs, two j atoms at
-            // a time (loads issued together), until one pair is in range
-            bool keep = false;
-            if (cand) {
-                const R px = (R)ox, py = (R)oy, pz = (R)oz;
-                const V4t* __restrict__ xj = xq + (size_t)my.j * CLUSTER;
-#pragma unroll 1
-                for (int j = 0; j < CLUSTER && !keep; j += 2) {
-                    V4t v[2];
-                    v[0] = xj[j];
-                    v[1] = xj[j + 1];
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const R qx = v[u].x + px, qy = v[u].y + py, qz = v[u].z + pz;
-                        const R thr = rc2 - (qx * qx + qy * qy + qz * qz);
-                        R m = fma(ax[0], qx, fma(ay[0], qy, fma(az[0], qz, an[0])));
-#pragma unroll
-                        for (int ii = 1; ii < CLUSTER; ++ii)
-                            m = fmin(m, fma(ax[ii], qx, fma(ay[ii], qy, fma(az[ii], qz, an[ii]))));
-                        keep = keep || m < thr;
-                    }
-                }
-            }
-            keepmask = __ballot_sync(0xffffffffu, keep);
-        } else {
-            // FP64 (half-rate arithmetic: idle lanes cost more than bookkeeping):
-            // the pending candidates four at a time, eight lanes (one j atom
-            // each) per candidate
-            const int slot = lane >> 3, jj = lane & 7;
-            unsigned todo = __ballot_sync(0xffffffffu, cand);
-            unsigned mine = 0u;
-            while (todo) {
-                // this lane's candidate: the (slot+1)-th lowest pending entry
-                unsigned x = todo;
-                if (slot >= 1) x &= x - 1u;
-                if (slot >= 2) x &= x - 1u;
-                if (slot >= 3) x &= x - 1u;
-                const bool valid = x != 0u;
-                const int sl = valid ? __ffs(x) - 1 : 0;
-                const int j = __shfl_sync(0xffffffffu, my.j, sl);
-                const R px = (R)__shfl_sync(0xffffffffu, ox, sl), py = (R)__shfl_sync(0xffffffffu, oy, sl),
-                        pz = (R)__shfl_sync(0xffffffffu, oz, sl);
-                const V4t vj = xq[j * CLUSTER + jj];
-                const R qx = vj.x + px, qy = vj.y + py, qz = vj.z + pz;
-                const R thr = rc2 - (qx * qx + qy * qy + qz * qz);
-                R m = fma(ax[0], qx, fma(ay[0], qy, fma(az[0], qz, an[0])));
-#pragma unroll
-                for (int ii = 1; ii < CLUSTER; ++ii)
-                    m = fmin(m, fma(ax[ii], qx, fma(ay[ii], qy, fma(az[ii], qz, an[ii]))));
-                const unsigned bal = __ballot_sync(0xffffffffu, valid && m < thr);
-                // lane L's own entry, if pending and among the four: its rank is its slot
-                const unsigned rank = __popc(todo & below);
-                if (((todo >> lane) & 1u) && rank < 4u && ((bal >> (8u * rank)) & 0xffu)) mine = 1u;
-                todo &= todo - 1u;
-                todo &= todo - 1u;
-                todo &= todo - 1u;
-                todo &= todo - 1u;
-            }
-            keepmask = __ballot_sync(0xffffffffu, mine != 0u);
-        }
-        if ((keepmask >> lane) & 1u) plist_in[L.start + kept + __popc(keepmask & below)] = my;
-        kept += __popc(keepmask);
-    }
-    if (lane == 0) {
-        ILRange r;
-        r.i = I; r.start = L.start; r.count = kept; r.pad = 0;
-        ilist_in[w] = r;
-    }
-}
-
-// Half prune (the 4 x 8 pair layout): the same box test, then each half of
-// the i cluster (atoms 0-3, 4-7) is tested on its own; an entry goes to the
-// list of every half that has an atom pair within the radius.  One lane per
-// outer entry, two j atoms at a time, stopping once both halves are found.
-// The outer range [start, start + count) of i cluster I owns the slots
-// [2 start + h count, 2 start + (h + 1) count) of the half list; item 2 w + h
-// of this launch describes half h (ILRange.pad = h).
-template <typename R>
-__device__ __forceinline__ void prune_half_dev(const PruneArgs<R>& A)
-{
-    using V4t = typename V4<R>::type;
-    if (!A.force && __uint_as_float(*A.disp) <= A.disp_thr2) return;   // self-pruning: the lists still hold
-    __shared__ float sh[27][6];
+    __shared__ float4 cand[PRUNE_WARPS][32];          // the entries to test: J's frame origin seen from I's, J
+    __shared__ unsigned kmask[2][HALF ? 2 : 1][W];    // kept entries of a round, per warp of the cluster (W > 1)
     for (int k = threadIdx.x; k < 27 * 6; k += blockDim.x) sh[k / 6][k % 6] = A.shifts.v[k / 6][k % 6];
     __syncthreads();
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // W == 1: the block's warps take a cluster each; W > 1: a block of W warps takes one
+    const int w = W == 1 ? (int)(blockIdx.x * (blockDim.x >> 5)) + wib : (int)blockIdx.x;
+    const int sub = W == 1 ? 0 : wib;
     if (w >= A.ncl) return;
     const unsigned below = (1u << lane) - 1u;
     const ILRange L = A.ilist[w];
     const int I = L.i;
-    const V4t* __restrict__ xq = A.xq;
-    if (A.snap && lane < CLUSTER) A.snap[I * CLUSTER + lane] = xq[I * CLUSTER + lane];
-    R ax[CLUSTER], ay[CLUSTER], az[CLUSTER], an[CLUSTER];   // -2 x_i and |x_i|^2
-#pragma unroll
-    for (int k = 0; k < CLUSTER; ++k) {
-        const V4t v = xq[I * CLUSTER + k];
-        ax[k] = (R)-2 * v.x; ay[k] = (R)-2 * v.y; az[k] = (R)-2 * v.z;
-        an[k] = v.x * v.x + v.y * v.y + v.z * v.z;
+    const float4* __restrict__ xf = A.xf;
+    if (sub == 0 && lane < CLUSTER) {
+        if (A.snap_d) A.snap_d[I * CLUSTER + lane] = A.xd[I * CLUSTER + lane];
+        else if (A.snap_f) A.snap_f[I * CLUSTER + lane] = xf[I * CLUSTER + lane];
     }
-    const float4 cI = A.centerf[I], ilo = A.cur_lo[I], ihi = A.cur_hi[I];
-    const R rc2 = (R)A.rcut2;
-    const long long out0 = 2LL * L.start, out1 = 2LL * L.start + L.count;
-    int kept0 = 0, kept1 = 0;
-    for (int base = 0; base < L.count; base += 32) {
-        const bool have = base + lane < L.count;
+    F32x2 ax[4], ay[4], az[4], an[4];   // -2 x_i and |x_i|^2 of atoms 2k, 2k + 1
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 u = xf[I * CLUSTER + 2 * k], v = xf[I * CLUSTER + 2 * k + 1];
+        ax[k] = pack2(-2.f * u.x, -2.f * v.x);
+        ay[k] = pack2(-2.f * u.y, -2.f * v.y);
+        az[k] = pack2(-2.f * u.z, -2.f * v.z);
+        an[k] = pack2(u.x * u.x + u.y * u.y + u.z * u.z, v.x * v.x + v.y * v.y + v.z * v.z);
+    }
+    const float4 cI = A.centerf[I];
+    const BoxF bi = box_decode(A.box[I]);
+    const float rc2 = A.rcut2;
+    const long long out0 = HALF ? 2LL * L.start : L.start, out1 = 2LL * L.start + L.count;
+    int kept0 = 0, kept1 = 0, buf = 0;
+    for (int base = 0; base < L.count; base += 32 * W) {
+        const int e = base + 32 * sub + lane;
+        const bool have = e < L.count;
         PairEntry my;
         my.j = I; my.shift = 13; my.mask = 0ull;
-        if (have) my = A.plist[L.start + base + lane];
-        const float4 cJ = A.centerf[my.j], jlo = A.cur_lo[my.j], jhi = A.cur_hi[my.j];
+        if (have) my = A.plist[L.start + e];
+        const BoxF bj = box_decode(A.box[my.j]);
         const float* s6 = sh[my.shift];
-        const float ox = -(((cI.x - cJ.x) - s6[0]) - s6[3]);
-        const float oy = -(((cI.y - cJ.y) - s6[1]) - s6[4]);
-        const float oz = -(((cI.z - cJ.z) - s6[2]) - s6[5]);
-        const float gx = fmaxf(0.f, fmaxf(jlo.x + ox - ihi.x, ilo.x - (jhi.x + ox)));
-        const float gy = fmaxf(0.f, fmaxf(jlo.y + oy - ihi.y, ilo.y - (jhi.y + oy)));
-        const float gz = fmaxf(0.f, fmaxf(jlo.z + oz - ihi.z, ilo.z - (jhi.z + oz)));
-        const bool cand = have && my.mask != 0ull && gx * gx + gy * gy + gz * gz < A.rcut2;
+        const float dx = fabsf((bi.x - bj.x) - s6[0]), dy = fabsf((bi.y - bj.y) - s6[1]),
+                    dz = fabsf((bi.z - bj.z) - s6[2]);
+        const float sx = bi.hx + bj.hx, sy = bi.hy + bj.hy, sz = bi.hz + bj.hz;
+        const float gx = fmaxf(0.f, dx - sx), gy = fmaxf(0.f, dy - sy), gz = fmaxf(0.f, dz - sz);
+        bool todo = have && my.mask != 0ull && gx * gx + gy * gy + gz * gz < rc2;
         bool k0 = false, k1 = false;
-        if (cand) {
-            const R px = (R)ox, py = (R)oy, pz = (R)oz;
-            const V4t* __restrict__ xj = xq + (size_t)my.j * CLUSTER;
-#pragma unroll 1
-            for (int j = 0; j < CLUSTER && !(k0 && k1); j += 2) {
-                V4t v[2];
-                v[0] = xj[j];
-                v[1] = xj[j + 1];
+        if (!HALF) {
+            // the face atoms towards each other along one axis: that far apart
+            // along it (+ the boxes' padding and their rounding to 1/64 A), at most the spans along the others
+            const float ux = fabsf(dx - sx) + 0.04f, uy = fabsf(dy - sy) + 0.04f, uz = fabsf(dz - sz) + 0.04f;
+            const float wx = (dx + sx) * (dx + sx), wy = (dy + sy) * (dy + sy), wz = (dz + sz) * (dz + sz);
+            const float far2 = fminf(ux * ux + wy + wz, fminf(wx + uy * uy + wz, wx + wy + uz * uz));
+            k0 = todo && far2 < rc2 && A.box_fine && bi.fine && bj.fine;
+            todo = todo && !k0;
+        }
+        const unsigned tb = __ballot_sync(0xffffffffu, todo);
+        const int rank = __popc(tb & below), n = __popc(tb);
+        if (todo) {
+            const float4 cJ = A.centerf[my.j];
+            cand[wib][rank] = make_float4(-(((cI.x - cJ.x) - s6[0]) - s6[3]), -(((cI.y - cJ.y) - s6[1]) - s6[4]),
+                                          -(((cI.z - cJ.z) - s6[2]) - s6[5]), __int_as_float(my.j));
+        }
+        __syncwarp();
+        for (int p = 0; p < n; p += 8) {
+            const float4 o = cand[wib][min(p + (lane >> 2), n - 1)];
+            const float4* __restrict__ xj = xf + (size_t)__float_as_int(o.w) * CLUSTER + 2 * (lane & 3);
+            float4 v[2];
+            v[0] = xj[0];
+            v[1] = xj[1];
+            bool h0 = false, h1 = false;
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const R qx = v[u].x + px, qy = v[u].y + py, qz = v[u].z + pz;
-                    const R thr = rc2 - (qx * qx + qy * qy + qz * qz);
-                    R m0 = fma(ax[0], qx, fma(ay[0], qy, fma(az[0], qz, an[0])));
-                    R m1 = fma(ax[4], qx, fma(ay[4], qy, fma(az[4], qz, an[4])));
+            for (int u = 0; u < 2; ++u) {
+                const float qx = v[u].x + o.x, qy = v[u].y + o.y, qz = v[u].z + o.z;
+                const float thr = rc2 - (qx * qx + qy * qy + qz * qz);
+                const F32x2 qx2 = pack2(qx, qx), qy2 = pack2(qy, qy), qz2 = pack2(qz, qz);
+                float m0 = 3.0e38f, m1 = 3.0e38f;
 #pragma unroll
-                    for (int ii = 1; ii < 4; ++ii) {
-                        m0 = fmin(m0, fma(ax[ii], qx, fma(ay[ii], qy, fma(az[ii], qz, an[ii]))));
-                        m1 = fmin(m1, fma(ax[ii + 4], qx, fma(ay[ii + 4], qy, fma(az[ii + 4], qz, an[ii + 4]))));
-                    }
-                    k0 = k0 || m0 < thr;
-                    k1 = k1 || m1 < thr;
+                for (int k = 0; k < 4; ++k) {
+                    const F32x2 d = fma2(ax[k], qx2, fma2(ay[k], qy2, fma2(az[k], qz2, an[k])));
+                    if (HALF && k >= 2) m1 = min_with2(m1, d);
+                    else m0 = min_with2(m0, d);
                 }
+                h0 = h0 || m0 < thr;
+                if (HALF) h1 = h1 || m1 < thr;
+            }
+            const unsigned b0 = __ballot_sync(0xffffffffu, h0), b1 = HALF ? __ballot_sync(0xffffffffu, h1) : 0u;
+            if (todo && (rank >> 3) == (p >> 3)) {
+                k0 = ((b0 >> (4 * (rank & 7))) & 0xfu) != 0u;
+                if (HALF) k1 = ((b1 >> (4 * (rank & 7))) & 0xfu) != 0u;
             }
         }
-        const unsigned b0 = __ballot_sync(0xffffffffu, k0), b1 = __ballot_sync(0xffffffffu, k1);
-        if (k0) A.plist_in[out0 + kept0 + __popc(b0 & below)] = my;
-        if (k1) A.plist_in[out1 + kept1 + __popc(b1 & below)] = my;
-        kept0 += __popc(b0);
-        kept1 += __popc(b1);
+        const unsigned m0 = __ballot_sync(0xffffffffu, k0), m1 = HALF ? __ballot_sync(0xffffffffu, k1) : 0u;
+        int off0 = kept0, off1 = kept1;
+        if (W == 1) {
+            kept0 += __popc(m0);
+            kept1 += __popc(m1);
+        } else {
+            if (lane == 0) {
+                kmask[buf][0][sub] = m0;
+                if (HALF) kmask[buf][HALF ? 1 : 0][sub] = m1;
+            }
+            __syncthreads();   // every warp of the block runs the same rounds
+#pragma unroll
+            for (int k = 0; k < W; ++k) {
+                const int c0 = __popc(kmask[buf][0][k]), c1 = HALF ? __popc(kmask[buf][HALF ? 1 : 0][k]) : 0;
+                if (k < sub) {
+                    off0 += c0;
+                    off1 += c1;
+                }
+                kept0 += c0;
+                kept1 += c1;
+            }
+            buf ^= 1;   // the other buffer next round: no second barrier
+        }
+        if (k0) A.plist_in[out0 + off0 + __popc(m0 & below)] = my;
+        if (HALF && k1) A.plist_in[out1 + off1 + __popc(m1 & below)] = my;
     }
-    if (lane == 0) {
+    if (lane == 0 && sub == 0) {
         ILRange r;
         r.i = I; r.start = (int)out0; r.count = kept0; r.pad = 0;
-        A.ilist_in[2 * w] = r;
-        r.start = (int)out1; r.count = kept1; r.pad = 1;
-        A.ilist_in[2 * w + 1] = r;
-    }
-}
-
-template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 3) k_prune_half(PruneArgs<R> A)
-{
-    prune_half_dev(A);
-}
-
-template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 3) k_prune_half_multi(const PruneArgs<R>* __restrict__ As)
-{
-    const PruneArgs<R>& A = As[blockIdx.z];
-    if ((int)blockIdx.x >= A.gx) return;
-    prune_half_dev(A);
-}
-
-template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 3) k_prune(PruneArgs<R> A)
-{
-    prune_dev(A);
-}
-
-template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 3) k_prune_multi(const PruneArgs<R>* __restrict__ As)
-{
-    const PruneArgs<R>& A = As[blockIdx.z];
-    if ((int)blockIdx.x >= A.gx) return;
-    prune_dev(A);
-}
-
-// Prune arguments for this rank's i clusters (ncl = 0: nothing to do).
-template <typename R>
-PruneArgs<R> make_prune_args(const Ctx& c)
-{
-    PruneArgs<R> A;
-    // a hair above the cutoff so working-precision rounding never drops a pair at r ~ rc
-    const double rc = c.p.cutoff + std::max(0.0, c.p.prune_margin) + 0.02;
-    for (int code = 0; code < 27; ++code) {
-        int sv[3] = {code % 3 - 1, (code / 3) % 3 - 1, code / 9 - 1};
-        for (int d = 0; d < 3; ++d) {
-            double v = sv[d] * c.box[d];
-            float hi = (float)v;
-            A.shifts.v[code][d] = hi;
-            A.shifts.v[code][3 + d] = (float)(v - (double)hi);
+        A.ilist_in[HALF ? 2 * w : w] = r;
+        if (HALF) {
+            r.start = (int)out1; r.count = kept1; r.pad = 1;
+            A.ilist_in[2 * w + 1] = r;
         }
     }
+}
+
+template <int W, bool HALF>
+__global__ void __launch_bounds__(W == 1 ? 256 : 32 * W, W == 1 ? 4 : 32 / W) k_prune(PruneArgs A)
+{
+    prune_dev<W, HALF>(A);
+}
+
+template <int W, bool HALF>
+__global__ void __launch_bounds__(W == 1 ? 256 : 32 * W, W == 1 ? 4 : 32 / W)
+    k_prune_multi(const PruneArgs* __restrict__ As)
+{
+    const PruneArgs& A = As[blockIdx.z];
+    if ((int)blockIdx.x >= A.gx) return;
+    prune_dev<W, HALF>(A);
+}
+
+// Warps per i cluster of a launch over ncl clusters: four where one each
+// leaves SMs idle.  2,780 atoms (372 clusters) 24 -> 14 us, 7,309 atoms (941)
+// 21 -> 14 us; at 3,241 clusters 25 -> 21 us alone, but the evaluation went
+// from 130 to 135 us (the side stream fills the idle issue slots), and at
+// 12,144 the prune itself from 44 to 57 us.
+void set_prune_warps(PruneArgs& A, long long ncl)
+{
+    A.warps = ncl < 2048 ? 4 : 1;
+    A.gx = A.warps == 1 ? grid_blocks((long long)A.ncl * 32, 256) : std::max(1, A.ncl);
+}
+
+// Padding of the boxes against the FP32 rounding of their absolute centres
+// and of the image offsets: 4e-7 of the longest edge covers it.
+static float box_pad(const Ctx& c)
+{
+    return 1e-3f + 4e-7f * (float)std::max(c.box[0], std::max(c.box[1], c.box[2]));
+}
+
+// Prune arguments for this rank's i clusters (ncl = 0: nothing to do);
+// half: write the half lists (item 2 w + h of this rank's range).
+PruneArgs make_prune_args(const Ctx& c, bool half)
+{
+    PruneArgs A;
+    // a hair above the cutoff so FP32 rounding never drops a pair at r ~ rc
+    const double rc = c.p.cutoff + std::max(0.0, c.p.prune_margin) + 0.02;
+    A.shifts = make_shift_table(c);
     long long lo, hi;
     cluster_share(c, lo, hi);   // this rank's i clusters
     A.ncl = (int)(hi - lo);
-    A.gx = grid_blocks((long long)A.ncl * 32, 256);
     A.gy = 1;
+    set_prune_warps(A, A.ncl);
     A.ilist = c.ilist.p + lo;
     A.plist = c.plist.p;
-    A.xq = reinterpret_cast<const typename V4<R>::type*>(sizeof(R) == 4 ? (const void*)c.xq_f.p : (const void*)c.xq_d.p);
+    A.xf = c.xq_f.p;
+    A.xd = c.xq_d.p;
     A.centerf = c.centerf.p;
-    A.cur_lo = c.cur_lo.p;
-    A.cur_hi = c.cur_hi.p;
+    A.box = c.cur_box.p;
+    A.box_fine = box_pad(c) < 0.002f ? 1 : 0;
     A.rcut2 = (float)(rc * rc);
-    A.ilist_in = c.ilist_in.p + lo;
-    A.plist_in = c.plist_in.p;
-    const bool selfp = self_pruning(c);
-    A.snap = selfp ? reinterpret_cast<typename V4<R>::type*>(c.xq_snap.p) : nullptr;
+    A.ilist_in = half ? c.ilist_h.p + 2 * lo : c.ilist_in.p + lo;
+    A.plist_in = half ? c.plist_h.p : c.plist_in.p;
+    const bool selfp = self_pruning(c), mixed = c.p.precision == MDF_PREC_MIXED;
+    A.snap_f = selfp && mixed ? reinterpret_cast<float4*>(c.xq_snap.p) : nullptr;
+    A.snap_d = selfp && !mixed ? reinterpret_cast<double4*>(c.xq_snap.p) : nullptr;
     A.disp = reinterpret_cast<const unsigned*>(c.scal.p + SCAL_DISP);
     const float half_margin = (float)(0.5 * std::max(0.0, c.p.prune_margin));
     A.disp_thr2 = half_margin * half_margin;
@@ -790,31 +772,41 @@ void ensure_half_lists(Ctx& c)
     c.plist_h.alloc(2 * (size_t)std::max<size_t>(c.plist.n, 1));
 }
 
-// Prune arguments writing the half lists (item 2 w + h of this rank's range).
-template <typename R>
-PruneArgs<R> make_prune_half_args(const Ctx& c)
+// A prune kernel's launch.  A self-pruning one mostly returns at once, but an SM
+// has to drain to change how much of its L1 is shared memory, and the driver's
+// choice for this kernel differs from the pair kernel's: asking for the pair
+// kernel's (72% of the L1, three blocks) took a step of 28k-atom dynamics from
+// 130 to 121 us.  A prune that does the work keeps the driver's choice, whose
+// larger L1 it needs (100k atoms 44 against 48 us).
+template <typename A>
+static void launch_prune(void (*kern)(A), A arg, dim3 grid, int threads, bool selfp, cudaStream_t s)
 {
-    PruneArgs<R> A = make_prune_args<R>(c);
-    long long lo, hi;
-    cluster_share(c, lo, hi);
-    A.ilist_in = c.ilist_h.p + 2 * lo;
-    A.plist_in = c.plist_h.p;
-    return A;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at.val.sharedMemCarveout = 72;
+    cfg.attrs = &at;
+    cfg.numAttrs = selfp ? 1 : 0;
+    MDF_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, arg));
 }
-template PruneArgs<float> make_prune_half_args<float>(const Ctx&);
-template PruneArgs<double> make_prune_half_args<double>(const Ctx&);
-template PruneArgs<float> make_prune_args<float>(const Ctx&);
-template PruneArgs<double> make_prune_args<double>(const Ctx&);
 
-template <typename R>
-void launch_prune_multi(const PruneArgs<R>* d_args, int nsys, int gx, bool half, cudaStream_t s)
+template <typename A>
+static void launch_prune_form(void (*w1)(A), void (*w1h)(A), void (*w4)(A), void (*w4h)(A), A arg, int warps, bool half,
+                              dim3 grid, bool selfp, cudaStream_t s)
 {
-    if (half) k_prune_half_multi<R><<<dim3(gx, 1, nsys), 256, 0, s>>>(d_args);
-    else k_prune_multi<R><<<dim3(gx, 1, nsys), 256, 0, s>>>(d_args);
-    MDF_CUDA_TRY(cudaGetLastError());
+    if (warps == 1) launch_prune(half ? w1h : w1, arg, grid, 256, selfp, s);
+    else launch_prune(half ? w4h : w4, arg, grid, 128, selfp, s);
 }
-template void launch_prune_multi<float>(const PruneArgs<float>*, int, int, bool, cudaStream_t);
-template void launch_prune_multi<double>(const PruneArgs<double>*, int, int, bool, cudaStream_t);
+
+// warps: the same in every system's arguments.
+void launch_prune_multi(const PruneArgs* d_args, int nsys, int gx, int warps, bool half, bool selfp, cudaStream_t s)
+{
+    launch_prune_form<const PruneArgs*>(k_prune_multi<1, false>, k_prune_multi<1, true>, k_prune_multi<4, false>,
+                                        k_prune_multi<4, true>, d_args, warps, half, dim3(gx, 1, nsys), selfp, s);
+}
 
 // whole_entries: build the 8 x 8 pruned list even in the half layout (the
 // adjoint walks whole entries); it also prunes unconditionally.
@@ -823,20 +815,10 @@ void prune_pairlist(Ctx& c, bool whole_entries)
     if (whole_entries) c.pruned_valid = false;   // a self-pruning launch prunes when the list is not valid
     const bool half = half_layout(c) && !whole_entries;
     if (half) ensure_half_lists(c);
-    if (c.p.precision == MDF_PREC_MIXED) {
-        const PruneArgs<float> A = half ? make_prune_half_args<float>(c) : make_prune_args<float>(c);
-        if (A.ncl > 0) {
-            if (half) k_prune_half<float><<<grid_of(A), 256, 0, c.stream>>>(A);
-            else k_prune<float><<<grid_of(A), 256, 0, c.stream>>>(A);
-        }
-    } else {
-        const PruneArgs<double> A = half ? make_prune_half_args<double>(c) : make_prune_args<double>(c);
-        if (A.ncl > 0) {
-            if (half) k_prune_half<double><<<grid_of(A), 256, 0, c.stream>>>(A);
-            else k_prune<double><<<grid_of(A), 256, 0, c.stream>>>(A);
-        }
-    }
-    MDF_CUDA_TRY(cudaGetLastError());
+    const PruneArgs A = make_prune_args(c, half);
+    if (A.ncl > 0)
+        launch_prune_form<PruneArgs>(k_prune<1, false>, k_prune<1, true>, k_prune<4, false>, k_prune<4, true>, A, A.warps,
+                                     half, grid_of(A), !A.force, c.stream);
     c.launches += 1;
     c.pruned_valid = true;
     c.pruned_half = half;
@@ -861,8 +843,9 @@ PackArgs<R> make_pack_args(const Ctx& c)
     A.center = c.center.p;
     for (int d = 0; d < 3; ++d) A.L[d] = c.box[d];
     A.xq = reinterpret_cast<typename V4<R>::type*>(sizeof(R) == 4 ? (void*)c.xq_f.p : (void*)c.xq_d.p);
-    A.cur_lo = c.cur_lo.p;
-    A.cur_hi = c.cur_hi.p;
+    A.box = c.cur_box.p;
+    A.box_pad = box_pad(c);
+    A.xf = c.xq_f.p;
     A.snap = self_pruning(c) ? reinterpret_cast<const typename V4<R>::type*>(c.xq_snap.p) : nullptr;
     A.disp = reinterpret_cast<unsigned*>(c.scal.p + SCAL_DISP);
     A.st = c.status.p;
@@ -1059,10 +1042,9 @@ void build_pairlist(Ctx& c)
         c.n_clusters = ncl;
         c.n_slots = ncl * CLUSTER;
         c.n_entries = c.h_build[1];
-        c.cur_lo.alloc(ncl);
-        c.cur_hi.alloc(ncl);
-        if (c.p.precision == MDF_PREC_MIXED) c.xq_f.alloc(c.n_slots);
-        else c.xq_d.alloc(c.n_slots);
+        c.cur_box.alloc(ncl);
+        c.xq_f.alloc(c.n_slots);
+        if (c.p.precision != MDF_PREC_MIXED) c.xq_d.alloc(c.n_slots);
         if (c.p.prune_every < 0)
             c.xq_snap.alloc((c.p.precision == MDF_PREC_MIXED ? sizeof(float4) : sizeof(double4)) * (size_t)c.n_slots);
         if (half_layout(c)) ensure_half_lists(c);   // sized here, not inside a later stream capture
