@@ -751,6 +751,8 @@ int mdf_create(const mdf_topology* top, const mdf_params* p, mdf_ctx** out)
         // also relies on exp(-alpha^2 r^2) vanishing at r^2 = 1e30
         if (!(std::isfinite(c.alpha) && c.alpha >= 1e-12))
             throw ApiError(MDF_ERR_INVALID, "Ewald alpha must be finite and >= 1e-12 (ewald_tol in (0, 0.5))");
+        if (c.p.precision == MDF_PREC_FP64 && c.p.semantics == MDF_SEM_PHYSICAL)
+            c.ewald_poly = make_ewald_poly(c.alpha, c.p.cutoff);
         upload_topology(c, top);
         if (!(c.box[0] > 0 && c.box[1] > 0 && c.box[2] > 0))
             throw ApiError(MDF_ERR_INVALID, "periodic box required");

@@ -446,8 +446,13 @@ void enqueue_multi(mdf_batch* b, const MultiArgs<R>& M, const MultiDev<R>& D, co
             launch_pairs_f32_multi(D.pf32, n, M.gx_pairs, M.threads, M.dyn_pairs, M.energy, M.use_switch, M.persist,
                                    M.half, M.lj_smem, M.parts, b->main);
         else
-            launch_pairs_f64_multi(D.p64, n, M.gx_pairs, M.threads, M.dyn_pairs, M.energy, M.use_switch, M.persist,
-                                   M.half, M.lj_smem, b->main);
+            for (int i = 0, j; i < n; i = j) {   // runs of systems with the same Ewald polynomials
+                for (j = i + 1; j < n && !memcmp(&M.p64[j].poly, &M.p64[i].poly, sizeof(EwaldPoly)); ++j) {
+                }
+                launch_pairs_f64_multi(D.p64 + i, j - i, M.gx_pairs, M.threads, M.dyn_pairs, M.energy, M.use_switch,
+                                       M.persist, M.half, M.lj_smem, M.p64[i].poly, b->main);
+                k += i > 0;
+            }
         ++k;
     }
     MDF_CUDA_TRY(cudaStreamWaitEvent(b->main, b->ev_join2, 0));

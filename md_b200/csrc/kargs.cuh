@@ -116,6 +116,7 @@ struct PairConstD {
     double rc2, alpha, two_a_spi;
     double inv_sw, rsw_inv, d30, d60;   // switch: x = r inv_sw - rsw_inv; dS/dr = x^2 (d30 + x (d60 + x d30))
     double uc6, uc12, rc;               // force-shifted LJ
+    double two_rc2;                     // 2 / rc^2 (argument of the Ewald polynomials)
 };
 
 struct ShiftTableD {
@@ -143,6 +144,7 @@ struct PairF64Args {
     unsigned long long* next;   // work counter of the persistent warps, zero at launch
     int persist;                // 1: persistent warps on the counter; 0: warp w takes item w
     int half;                   // lists are half entries (the 4 x 8 kernel)
+    EwaldPoly poly;
     unsigned* st;
 };
 
@@ -363,7 +365,7 @@ void launch_pairs_f32_multi(const PairF32Args* d_args, int nsys, int gx, int thr
 template <typename R> PairArgs<R> make_pair_args(const Ctx& c, bool count);
 PairF64Args make_pair_f64_args(const Ctx& c, size_t* dyn);
 void launch_pairs_f64_multi(const PairF64Args* d_args, int nsys, int gx, int threads, size_t dyn, bool energy,
-                            bool use_switch, bool persist, bool half, bool lj_smem, cudaStream_t s);
+                            bool use_switch, bool persist, bool half, bool lj_smem, const EwaldPoly& poly, cudaStream_t s);
 int pair_threads(const Ctx& c);
 int pair_split(long long nlist);
 // 2^split items per list, one warp each.

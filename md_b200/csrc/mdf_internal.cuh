@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/mdf.h"
+#include "ewald_poly.hpp"
 
 namespace mdf {
 
@@ -133,6 +134,7 @@ struct Ctx {
     DevBuf<double4> ljAB4_d;       // the same in FP64 (FP64 PHYSICAL pair kernel)
     DevBuf<double2> lj14AB;    // same indexing, 1-4 tables
     DevBuf<int> ljvalid;       // [(ntypes+1)^2] nb != 0
+    EwaldPoly ewald_poly{};    // FP64 PHYSICAL contexts
     int ntp = 0;               // ntypes + 1 (padding type appended)
     int n_ljpair = 0;
     std::vector<int> h_nb_index;         // [ntypes^2] NONBONDED_PARM_INDEX (host copy)
