@@ -266,6 +266,13 @@ void upload_topology(Ctx& c, const mdf_topology* t)
     c.ntp = t->ntypes + 1;
     for (int i = 0; i < c.N; ++i)
         if (t->type[i] < 0 || t->type[i] >= t->ntypes) throw ApiError(MDF_ERR_INVALID, "atom type out of range");
+    {
+        std::vector<int> n(t->ntypes, 0);
+        for (int i = 0; i < c.N; ++i) ++n[t->type[i]];
+        c.hot_type[0] = (int)(std::max_element(n.begin(), n.end()) - n.begin());
+        n[c.hot_type[0]] = -1;
+        c.hot_type[1] = t->ntypes > 1 ? (int)(std::max_element(n.begin(), n.end()) - n.begin()) : c.hot_type[0];
+    }
     c.n_ljpair = t->n_ljpair;
     c.h_nb_index.assign(t->nb_index, t->nb_index + (size_t)c.ntypes * c.ntypes);
     for (int i = 0; i < c.ntypes; ++i)
@@ -816,6 +823,8 @@ void mdf_destroy(mdf_ctx* ctx)
             cudaStreamDestroy(cs);
         }
     c.d_build.release();
+    c.adj_v.release(); c.adj_vs_f.release(); c.adj_vs_d.release(); c.adj_dq_slot.release(); c.adj_dq_atom.release();
+    c.adj_dab.release(); c.adj_dq.release(); c.adj_qgrid.release(); c.adj_cgrid.release(); c.adj_rgrid.release();
     if (c.md_exec) cudaGraphExecDestroy(c.md_exec);
     if (c.md_graph) cudaGraphDestroy(c.md_graph);
     if (c.md_host) cudaFreeHost(c.md_host);

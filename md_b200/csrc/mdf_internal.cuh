@@ -134,6 +134,7 @@ struct Ctx {
     DevBuf<double4> ljAB4_d;       // the same in FP64 (FP64 PHYSICAL pair kernel)
     DevBuf<double2> lj14AB;    // same indexing, 1-4 tables
     DevBuf<int> ljvalid;       // [(ntypes+1)^2] nb != 0
+    int hot_type[2] = {0, 0};  // the two most frequent atom types
     EwaldPoly ewald_poly{};    // FP64 PHYSICAL contexts
     int ntp = 0;               // ntypes + 1 (padding type appended)
     int n_ljpair = 0;
@@ -238,6 +239,8 @@ struct Ctx {
     DevBuf<unsigned long long> adj_dq_slot, adj_dq_atom;   // fixed-point dL/dq
     DevBuf<double> adj_dab;              // [2 n_ljpair] dL/dA | dL/dB
     DevBuf<double> adj_dq;               // [N] dL/dq out
+    DevBuf<unsigned long long> adj_qgrid;   // charge grid | dipole grid
+    DevBuf<unsigned char> adj_cgrid, adj_rgrid;   // their half-complex grids and potentials
 
     // dynamics and minimiser (md.cu)
     DevBuf<double> md_v;                 // [3N] velocities, A/ps
