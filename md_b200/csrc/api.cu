@@ -358,6 +358,19 @@ void upload_topology(Ctx& c, const mdf_topology* t)
         if (!sex.count(pr)) throw ApiError(MDF_ERR_INVALID, "1-4 pair missing from the exclusion list");
     c.excl_pairs.upload(ex.data(), ex.size(), s);
     c.excl_is14.upload(is14.data(), is14.size(), s);
+    if (c.n_excl > 0) {
+        std::vector<int> off(c.N + 1, 0), nb(ex.size());
+        for (int a : ex) ++off[a + 1];
+        for (int i = 0; i < c.N; ++i) off[i + 1] += off[i];
+        std::vector<int> at(off.begin(), off.end() - 1);
+        for (size_t i = 0; i < ex.size(); i += 2) {
+            nb[at[ex[i]]++] = ex[i + 1];
+            nb[at[ex[i + 1]]++] = ex[i];
+        }
+        c.ex_off.upload(off.data(), off.size(), s);
+        c.ex_nb.upload(nb.data(), nb.size(), s);
+        MDF_CUDA_TRY(cudaStreamSynchronize(s));
+    }
     {
         std::vector<int> p(2 * (size_t)c.n_14);
         std::vector<double2> sc(c.n_14);
@@ -794,11 +807,11 @@ void mdf_destroy(mdf_ctx* ctx)
     c.bond_atoms.release(); c.ub_atoms.release(); c.angle_atoms.release(); c.dih_atoms.release();
     c.imp_atoms.release(); c.cmap_atoms.release(); c.cmap_set.release(); c.bond_par.release(); c.ub_par.release();
     c.angle_par.release(); c.imp_par.release(); c.dih_par.release(); c.cmap_coeff.release();
-    c.excl_pairs.release(); c.pairs14.release(); c.p14_scale.release(); c.excl_is14.release();
+    c.excl_pairs.release(); c.pairs14.release(); c.p14_scale.release(); c.excl_is14.release(); c.ex_off.release(); c.ex_nb.release();
     c.xyz.release(); c.atom_col.release(); c.col_count.release(); c.col_start.release(); c.col_cstart.release();
     c.col_atoms.release(); c.slot_atom.release(); c.atom_slot.release(); c.slot_type.release(); c.center.release(); c.centerf.release();
     c.bb_lo.release(); c.bb_hi.release(); c.xq_f.release(); c.xq_d.release(); c.cluster_col.release();
-    c.ilist.release(); c.plist.release(); c.scan_tmp.release(); c.f_slot.release();
+    c.ilist.release(); c.plist.release(); c.f_slot.release();
     c.plist_in.release(); c.ilist_in.release(); c.cur_box.release(); c.xq_snap.release();
     c.q_slab.release(); c.pme_slab.release(); c.pme_send.release(); c.pme_recv.release(); c.pme_rslab.release();
     c.f_stage.release(); c.f_mine.release(); c.f_out_blk.release(); c.f_out_all.release();

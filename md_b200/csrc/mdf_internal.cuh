@@ -134,6 +134,7 @@ struct Ctx {
     DevBuf<double4> ljAB4_d;       // the same in FP64 (FP64 PHYSICAL pair kernel)
     DevBuf<double2> lj14AB;    // same indexing, 1-4 tables
     DevBuf<int> ljvalid;       // [(ntypes+1)^2] nb != 0
+    DevBuf<int> ex_off, ex_nb; // each atom's excluded partners: ex_nb[ex_off[a] .. ex_off[a + 1])
     int hot_type[2] = {0, 0};  // the two most frequent atom types
     EwaldPoly ewald_poly{};    // FP64 PHYSICAL contexts
     int ntp = 0;               // ntypes + 1 (padding type appended)
@@ -166,7 +167,7 @@ struct Ctx {
     int ncol_x = 0, ncol_y = 0, ncols = 0;
     int n_clusters = 0, n_slots = 0;
     bool have_list = false;
-    DevBuf<int> atom_col;          // [N]
+    DevBuf<int2> atom_col;          // [N]
     DevBuf<int> col_count, col_start, col_cstart;   // [ncols + 1]
     DevBuf<int> col_atoms;         // [N] atoms bucketed by column
     DevBuf<int> slot_atom;         // [n_slots]
@@ -191,7 +192,6 @@ struct Ctx {
     DevBuf<unsigned char> xq_snap; // self-pruning mode: the cluster-frame positions of the last prune, per slot
     int since_prune = 0;
     bool pruned_valid = false;
-    DevBuf<int> scan_tmp;
     DevBuf<int> d_build;           // [4] list entries claimed by the search
     int* h_build = nullptr;        // pinned: cluster count, entry count, status of the last build
 
