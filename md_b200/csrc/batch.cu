@@ -205,7 +205,7 @@ struct MultiArgs {
     std::vector<FinalizeArgs> fin;
     // block maps of the kernels whose per-system grids differ most between
     // systems (one entry per block actually needed: no idle blocks)
-    std::vector<int2> map_pack, map_zero, map_spread, map_z, map_y, map_x, map_gather, map_fin;
+    std::vector<int2> map_pack, map_zero, map_spread, map_z[2], map_y[2], map_x[2], map_gather, map_fin;
     FFTChainMax fm{};
     int gx_prune = 0, gx_pairs = 0, gx_excl = 0, gx_14 = 0, gx_bonded = 0;
     size_t dyn_pairs = 0;
@@ -308,12 +308,13 @@ MultiDev<R> prepare_multi(mdf_batch* b, uint32_t flags, MultiArgs<R>& M, double*
         M.x.push_back(F.x);
         M.yi.push_back(F.yi);
         M.zi.push_back(F.zi);
-        add_blocks(M.map_z, s, F.zf.gx, F.zf.gy);
-        add_blocks(M.map_y, s, F.yf.gx, F.yf.gy);
-        add_blocks(M.map_x, s, F.x.gx, F.x.gy);
-        M.fm.smz = std::max(M.fm.smz, F.smz);
-        M.fm.smy = std::max(M.fm.smy, F.smy);
-        M.fm.smx = std::max(M.fm.smx, F.smx);
+        const int iz = F.zf.d.r[0] ? 1 : 0, iy = F.yf.d.r[0] ? 1 : 0, ix = F.x.d.r[0] ? 1 : 0;
+        add_blocks(M.map_z[iz], s, F.zf.gx, F.zf.gy);
+        add_blocks(M.map_y[iy], s, F.yf.gx, F.yf.gy);
+        add_blocks(M.map_x[ix], s, F.x.gx, F.x.gy);
+        M.fm.smz[iz] = std::max(M.fm.smz[iz], F.smz);
+        M.fm.smy[iy] = std::max(M.fm.smy[iy], F.smy);
+        M.fm.smx[ix] = std::max(M.fm.smx[ix], F.smx);
         M.gather.push_back(make_gather_args<R>(c));
         // forces straight into the batch's concatenated device buffer
         M.fin.push_back(make_finalize_args(c, d_forces + b->off[s]));
@@ -360,8 +361,9 @@ MultiDev<R> prepare_multi(mdf_batch* b, uint32_t flags, MultiArgs<R>& M, double*
                          arr_bytes(M.spread) + arr_bytes(M.zf) + arr_bytes(M.yf) + arr_bytes(M.x) +
                          arr_bytes(M.yi) + arr_bytes(M.zi) + arr_bytes(M.gather) + arr_bytes(M.fin) +
                          arr_bytes(M.map_pack) + arr_bytes(M.map_zero) + arr_bytes(M.map_spread) +
-                         arr_bytes(M.map_z) + arr_bytes(M.map_y) + arr_bytes(M.map_x) + arr_bytes(M.map_gather) +
-                         arr_bytes(M.map_fin);
+                         arr_bytes(M.map_z[0]) + arr_bytes(M.map_y[0]) + arr_bytes(M.map_x[0]) +
+                         arr_bytes(M.map_z[1]) + arr_bytes(M.map_y[1]) + arr_bytes(M.map_x[1]) +
+                         arr_bytes(M.map_gather) + arr_bytes(M.map_fin);
     std::vector<unsigned char> host(total);
     args.alloc(total);
     size_t off = 0;
@@ -399,9 +401,11 @@ MultiDev<R> prepare_multi(mdf_batch* b, uint32_t flags, MultiArgs<R>& M, double*
     putmap(M.map_spread, D.spread_m);
     putmap(M.map_gather, D.gather_m);
     putmap(M.map_fin, D.fin_m);
-    putmap(M.map_z, D.fft.mz);
-    putmap(M.map_y, D.fft.my);
-    putmap(M.map_x, D.fft.mx);
+    for (int i = 0; i < 2; ++i) {
+        putmap(M.map_z[i], D.fft.mz[i]);
+        putmap(M.map_y[i], D.fft.my[i]);
+        putmap(M.map_x[i], D.fft.mx[i]);
+    }
     MDF_CUDA_TRY(cudaMemcpyAsync(args.p, host.data(), total, cudaMemcpyHostToDevice, b->main));
     MDF_CUDA_TRY(cudaStreamSynchronize(b->main));
     return D;
@@ -432,7 +436,9 @@ void enqueue_multi(mdf_batch* b, const MultiArgs<R>& M, const MultiDev<R>& D, co
     k += M.gx_bonded > 0;
     launch_pme_multi<R>(D.zero, D.zero_m, D.spread, D.spread_m, D.fft, M.fm, D.gather, D.gather_m, M.energy,
                         b->side);
-    k += 8;   // grid clear, spread, five FFT passes, gather
+    k += 3;   // grid clear, spread, gather
+    for (int i = 0; i < 2; ++i)   // the FFT passes of either form that have blocks
+        k += 2 * (D.fft.mz[i].n > 0) + 2 * (D.fft.my[i].n > 0) + (D.fft.mx[i].n > 0);
     MDF_CUDA_TRY(cudaEventRecord(b->ev_join2, b->side));
     // main stream: pack, prune, pair kernel
     launch_pack_multi<R>(D.pack, D.pack_m, b->main);

@@ -266,6 +266,7 @@ struct FFTDesc {
     int ns[12];
     int toff[12];
     int ntab;
+    int r[3];         // register radices (fft_regs.cuh); r[0] = 0: none, the table-driven passes
 };
 
 struct ConvParams {
@@ -365,12 +366,13 @@ struct FFTChainDev {
     const FFTXArgs<R>* x;
     const FFTYArgs<R>* yi;
     const FFTZArgs<R>* zi;
-    BlockMap mz, my, mx;   // the blocks of the z, y and x passes (forward and inverse share them)
+    // the blocks of the z, y and x passes (forward and inverse share them): [0] table-driven, [1] register radices
+    BlockMap mz[2], my[2], mx[2];
 };
 
 // ... and the largest shared memory of each pass over the systems.
 struct FFTChainMax {
-    size_t smz, smy, smx;
+    size_t smz[2], smy[2], smx[2];
 };
 
 // --------------------------------------------------------------- finalize

@@ -111,6 +111,7 @@ struct FFTPlan1D {
     int ns[12];     // product of the radices before stage s
     int toff[12];   // offset of stage s in the per-butterfly index table
     int ntab = 0;   // entries of the index table
+    int r[3] = {0, 0, 0};   // register radices (fft_regs.cuh)
 };
 
 // --------------------------------------------------------------- context
@@ -227,8 +228,8 @@ struct Ctx {
     DevBuf<float2> tw_f[3];
     FFTPlan1D plan[3];
     DevBuf<int2> fft_tab[3];             // per-butterfly (twiddle step, output index) per dimension
-    DevBuf<float> infl_f;                // influence function [ky][kz][kx] (mixed)
-    DevBuf<double> infl_d;               // influence function [ky][kz][kx] (FP64 / reference solve)
+    DevBuf<float> infl_f;                // influence function, laid out for the x pass (mixed)
+    DevBuf<double> infl_d;               // the same (FP64 / reference solve)
     DevBuf<double> mvec[3];              // m_d = signed frequency / L_d per grid index
     bool have_pme_ref = false;           // forces_pme_ref holds the reference chain's forces
 

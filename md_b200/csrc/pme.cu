@@ -10,10 +10,10 @@
 // its gather (:576-653).  The reference discards those forces; they are
 // returned separately for parity checks.
 //
-// FFT: mixed-radix Stockham autosort in shared memory (radix 4/2/3/5 and a
-// generic small-prime butterfly).  Every butterfly's twiddle step and output
-// index come from a table built on the host, so the passes do no integer
-// division.  One kernel per dimension:
+// FFT: register radices for lengths that are products of two or three of them
+// (fft_regs.cuh); other lengths run the mixed-radix Stockham passes here (radix
+// 4/2/3/5 and a generic small-prime butterfly, twiddle step and output index of
+// every butterfly from a table built on the host).  One kernel per dimension:
 //   z: real -> half complex, two real lines packed per complex transform
 //   y: complex, LP consecutive kz columns per block (coalesced along kz)
 //   x: complex forward, convolution with the precomputed influence function
@@ -27,34 +27,12 @@
 #include <string>
 #include <vector>
 
+#include "fft_regs.cuh"
 #include "kargs.cuh"
 #include "mdf_device.cuh"
 #include "mdf_internal.cuh"
 
 namespace mdf {
-
-template <typename R> struct CT;
-template <> struct CT<float> { using type = float2; };
-template <> struct CT<double> { using type = double2; };
-
-constexpr int FFT_THREADS = 128;
-
-
-template <typename C>
-__device__ __forceinline__ C cmul(C a, C b)
-{
-    C r;
-    r.x = a.x * b.x - a.y * b.y;
-    r.y = a.x * b.y + a.y * b.x;
-    return r;
-}
-
-template <typename C>
-__device__ __forceinline__ C cconj(C a)
-{
-    a.y = -a.y;
-    return a;
-}
 
 // In-place DFT of v[0..R-1]; forward uses W = exp(-2 pi i / R).
 template <typename C, typename R>
@@ -435,6 +413,81 @@ __global__ void __launch_bounds__(FFT_THREADS, 8) k_fft_x_conv_multi(const FFTXA
     fft_x_conv_dev<R, ENERGY>(A, m.y % A.gx, m.y / A.gx);
 }
 
+// The register-radix passes (fft_regs.cuh), same launch forms.
+template <typename R>
+__global__ void __launch_bounds__(FFT_THREADS) k_fftr_z_r2c(FFTZArgs<R> A) { regs_z_r2c_dev(A, blockIdx.x); }
+template <typename R>
+__global__ void __launch_bounds__(FFT_THREADS) k_fftr_z_c2r(FFTZArgs<R> A) { regs_z_c2r_dev(A, blockIdx.x); }
+template <typename R, bool INV>
+__global__ void __launch_bounds__(FFT_THREADS) k_fftr_y(FFTYArgs<R> A) { regs_y_dev<R, INV>(A, blockIdx.x, blockIdx.y); }
+template <typename R, bool ENERGY>
+__global__ void __launch_bounds__(FFT_THREADS) k_fftr_x_conv(FFTXArgs<R> A)
+{
+    regs_x_conv_dev<R, ENERGY>(A, blockIdx.x, blockIdx.y);
+}
+template <typename R>
+__global__ void __launch_bounds__(FFT_THREADS) k_fftr_z_r2c_multi(const FFTZArgs<R>* __restrict__ As,
+                                                                  const int2* __restrict__ bmap)
+{
+    const int2 m = bmap[blockIdx.x];
+    regs_z_r2c_dev(As[m.x], m.y);
+}
+template <typename R>
+__global__ void __launch_bounds__(FFT_THREADS) k_fftr_z_c2r_multi(const FFTZArgs<R>* __restrict__ As,
+                                                                  const int2* __restrict__ bmap)
+{
+    const int2 m = bmap[blockIdx.x];
+    regs_z_c2r_dev(As[m.x], m.y);
+}
+template <typename R, bool INV>
+__global__ void __launch_bounds__(FFT_THREADS) k_fftr_y_multi(const FFTYArgs<R>* __restrict__ As,
+                                                              const int2* __restrict__ bmap)
+{
+    const int2 m = bmap[blockIdx.x];
+    const FFTYArgs<R>& A = As[m.x];
+    regs_y_dev<R, INV>(A, m.y % A.gx, m.y / A.gx);
+}
+template <typename R, bool ENERGY>
+__global__ void __launch_bounds__(FFT_THREADS) k_fftr_x_conv_multi(const FFTXArgs<R>* __restrict__ As,
+                                                                   const int2* __restrict__ bmap)
+{
+    const int2 m = bmap[blockIdx.x];
+    const FFTXArgs<R>& A = As[m.x];
+    regs_x_conv_dev<R, ENERGY>(A, m.y % A.gx, m.y / A.gx);
+}
+
+// One system's passes, each in the form its length has (d.r[0] != 0: register radices).
+template <typename R>
+static void launch_z_r2c(const FFTZArgs<R>& A, size_t sm, cudaStream_t s)
+{
+    if (A.d.r[0]) k_fftr_z_r2c<R><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+    else k_fft_z_r2c<R><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+}
+template <typename R>
+static void launch_z_c2r(const FFTZArgs<R>& A, size_t sm, cudaStream_t s)
+{
+    if (A.d.r[0]) k_fftr_z_c2r<R><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+    else k_fft_z_c2r<R><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+}
+template <typename R>
+static void launch_y(const FFTYArgs<R>& A, size_t sm, cudaStream_t s)
+{
+    if (!A.d.r[0]) k_fft_y<R><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+    else if (A.inverse) k_fftr_y<R, true><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+    else k_fftr_y<R, false><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+}
+template <typename R>
+static void launch_x_conv(const FFTXArgs<R>& A, bool energy, size_t sm, cudaStream_t s)
+{
+    if (A.d.r[0]) {
+        if (energy) k_fftr_x_conv<R, true><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+        else k_fftr_x_conv<R, false><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+    } else {
+        if (energy) k_fft_x_conv<R, true><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+        else k_fft_x_conv<R, false><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+    }
+}
+
 // ------------------------------------------------------ spread / gather
 // Cardinal B-spline of order 4: th[j] = M4(w + 3 - j), placed at base-1+j.
 template <typename R>
@@ -785,6 +838,7 @@ static FFTPlan1D make_plan(int n, std::vector<int2>& tab)
         Ns *= R;
     }
     p.ntab = (int)tab.size();
+    fft_radices(n, p.r);
     return p;
 }
 
@@ -799,6 +853,7 @@ static FFTDesc to_desc(const FFTPlan1D& p)
         d.toff[i] = i < p.nstages ? p.toff[i] : 0;
     }
     d.ntab = p.ntab;
+    for (int i = 0; i < 3; ++i) d.r[i] = p.r[i];
     return d;
 }
 
@@ -842,6 +897,41 @@ static int lines_per_block(const FFTPlan1D& p, size_t csize, int cap = 0)
 static size_t fft_smem(const FFTPlan1D& p, size_t csize, int lp)
 {
     return csize * ((size_t)p.n + 2 * (size_t)lp * p.n) + sizeof(int2) * (size_t)p.ntab;
+}
+
+// Lines per block and shared memory of a register-radix pass over nlines lines
+// (rows blocks of them along the other dimension): mdf_params.fft_lines, or for
+// 0 up to 16 lines such that the stages' tasks fill the threads, the last block
+// of a row is not mostly empty, rows x blocks covers the SMs twice where the
+// grid allows it, and neighbouring lines make 32-byte reads or longer.
+static int regs_lines(const FFTPlan1D& p, size_t csize, int cap, long long nlines, long long rows, bool contiguous)
+{
+    const int fit = (int)std::max<long long>(1, std::min<long long>(nlines, (long long)((46 * 1024 - csize * p.n) / (2 * csize * p.n))));
+    if (cap == 1 || cap == 2 || cap == 4 || cap == 8 || cap == 16 || cap == 32) return std::min(cap, fit);
+    int best = 1;
+    double score = -1.0;
+    for (int lp = 1; lp <= std::min(16, fit); ++lp) {
+        double s = 1.0;
+        for (int r : {p.r[0], p.r[2]}) {
+            const int tasks = lp * (p.n / r);
+            s *= (double)tasks / (((tasks + FFT_THREADS - 1) / FFT_THREADS) * FFT_THREADS);
+        }
+        s = std::sqrt(s);
+        const long long blocks = (nlines + lp - 1) / lp;
+        s *= (double)nlines / (double)(blocks * lp);
+        s *= std::min(1.0, 0.5 + 0.5 * (double)(blocks * rows) / 296.0);
+        if (!contiguous) s *= std::min(1.0, 0.4 + 0.6 * (double)(lp * csize) / 64.0);
+        if (s > score + 1e-9) {
+            score = s;
+            best = lp;
+        }
+    }
+    return best;
+}
+
+static size_t regs_smem(const FFTPlan1D& p, size_t csize, int lp)
+{
+    return csize * ((size_t)p.n + 2 * (size_t)lp * p.n);
 }
 
 static int ilog2(int v)
@@ -931,7 +1021,9 @@ void setup_pme(Ctx& c)
             c.tw_d[d].upload(tw.data(), K, c.stream);
         }
     }
-    // influence function, laid out [ky][kz][kx] (the x pass reads lines along kx)
+    // influence function, laid out as the x pass reads it: [ky][kx][kz] with
+    // register radices, else [ky][kz][kx]
+    const bool kx_major = c.plan[0].r[0] != 0;
     std::vector<double> infl((size_t)K1 * Kc * K0);
     const double V = c.box[0] * c.box[1] * c.box[2];
     for (int ky = 0; ky < K1; ++ky) {
@@ -959,7 +1051,7 @@ void setup_pme(Ctx& c)
                         v = influence * b_corr * (1.0 / (double)ntot);
                     }
                 }
-                infl[((size_t)ky * Kc + kz) * K0 + kx] = v;
+                infl[kx_major ? ((size_t)ky * K0 + kx) * Kc + kz : ((size_t)ky * Kc + kz) * K0 + kx] = v;
             }
     }
     if (mixed) {
@@ -1013,9 +1105,11 @@ FFTChain<R> make_fft_chain(const Ctx& c, bool energy)
     const bool ref = c.p.semantics == MDF_SEM_REFERENCE;
     const int K0 = c.K[0], K1 = c.K[1], Kc = c.K[2] / 2 + 1;
     // z forward (real -> half complex) and z inverse share a geometry
-    const int LPz = lines_per_block(c.plan[2], sizeof(C), c.p.fft_lines);
-    F.smz = fft_smem(c.plan[2], sizeof(C), LPz);
     const int nlines = K0 * K1;
+    const bool rz = c.plan[2].r[0] != 0, ry = c.plan[1].r[0] != 0, rx = c.plan[0].r[0] != 0;
+    const int LPz = rz ? regs_lines(c.plan[2], sizeof(C), c.p.fft_lines, (nlines + 1) / 2, 1, true)
+                       : lines_per_block(c.plan[2], sizeof(C), c.p.fft_lines);
+    F.smz = rz ? regs_smem(c.plan[2], sizeof(C), LPz) : fft_smem(c.plan[2], sizeof(C), LPz);
     F.zf.gx = (nlines + 2 * LPz - 1) / (2 * LPz);
     F.zf.gy = 1;
     F.zf.qgrid = c.qgrid.p;
@@ -1028,8 +1122,9 @@ FFTChain<R> make_fft_chain(const Ctx& c, bool energy)
     F.zf.LP = LPz;
     F.zi = F.zf;
     // y forward / inverse
-    const int LPy = lines_per_block(c.plan[1], sizeof(C), c.p.fft_lines);
-    F.smy = fft_smem(c.plan[1], sizeof(C), LPy);
+    const int LPy = ry ? regs_lines(c.plan[1], sizeof(C), c.p.fft_lines, Kc, K0, false)
+                       : lines_per_block(c.plan[1], sizeof(C), c.p.fft_lines);
+    F.smy = ry ? regs_smem(c.plan[1], sizeof(C), LPy) : fft_smem(c.plan[1], sizeof(C), LPy);
     F.yf.gx = (Kc + LPy - 1) / LPy;
     F.yf.gy = K0;
     F.yf.cgrid = B.cg;
@@ -1043,8 +1138,9 @@ FFTChain<R> make_fft_chain(const Ctx& c, bool energy)
     F.yi = F.yf;
     F.yi.inverse = 1;
     // x forward + convolution + x inverse
-    const int LP = lines_per_block(c.plan[0], sizeof(C), c.p.fft_lines);
-    F.smx = fft_smem(c.plan[0], sizeof(C), LP);
+    const int LP = rx ? regs_lines(c.plan[0], sizeof(C), c.p.fft_lines, Kc, K1, false)
+                      : lines_per_block(c.plan[0], sizeof(C), c.p.fft_lines);
+    F.smx = rx ? regs_smem(c.plan[0], sizeof(C), LP) : fft_smem(c.plan[0], sizeof(C), LP);
     F.x.gx = (Kc + LP - 1) / LP;
     F.x.gy = K1;
     F.x.cgrid = B.cg;
@@ -1074,12 +1170,11 @@ template <typename R>
 static void conv_chain(Ctx& c, const PmeBufs<R>&, bool energy)
 {
     const FFTChain<R> F = make_fft_chain<R>(c, energy);
-    k_fft_z_r2c<R><<<grid_of(F.zf), FFT_THREADS, F.smz, c.stream>>>(F.zf);
-    k_fft_y<R><<<grid_of(F.yf), FFT_THREADS, F.smy, c.stream>>>(F.yf);
-    if (energy) k_fft_x_conv<R, true><<<grid_of(F.x), FFT_THREADS, F.smx, c.stream>>>(F.x);
-    else k_fft_x_conv<R, false><<<grid_of(F.x), FFT_THREADS, F.smx, c.stream>>>(F.x);
-    k_fft_y<R><<<grid_of(F.yi), FFT_THREADS, F.smy, c.stream>>>(F.yi);
-    k_fft_z_c2r<R><<<grid_of(F.zi), FFT_THREADS, F.smz, c.stream>>>(F.zi);
+    launch_z_r2c(F.zf, F.smz, c.stream);
+    launch_y(F.yf, F.smy, c.stream);
+    launch_x_conv(F.x, energy, F.smx, c.stream);
+    launch_y(F.yi, F.smy, c.stream);
+    launch_z_c2r(F.zi, F.smz, c.stream);
 }
 
 // Many systems' FFT chains, one launch per pass (each struct array holds one
@@ -1088,14 +1183,22 @@ static void conv_chain(Ctx& c, const PmeBufs<R>&, bool energy)
 template <typename R>
 void launch_fft_chain_multi(const FFTChainDev<R>& D, const FFTChainMax& M, bool energy, cudaStream_t s)
 {
-    if (D.mz.n > 0) k_fft_z_r2c_multi<R><<<D.mz.n, FFT_THREADS, M.smz, s>>>(D.zf, D.mz.map);
-    if (D.my.n > 0) k_fft_y_multi<R><<<D.my.n, FFT_THREADS, M.smy, s>>>(D.yf, D.my.map);
-    if (D.mx.n > 0) {
-        if (energy) k_fft_x_conv_multi<R, true><<<D.mx.n, FFT_THREADS, M.smx, s>>>(D.x, D.mx.map);
-        else k_fft_x_conv_multi<R, false><<<D.mx.n, FFT_THREADS, M.smx, s>>>(D.x, D.mx.map);
+    if (D.mz[0].n > 0) k_fft_z_r2c_multi<R><<<D.mz[0].n, FFT_THREADS, M.smz[0], s>>>(D.zf, D.mz[0].map);
+    if (D.mz[1].n > 0) k_fftr_z_r2c_multi<R><<<D.mz[1].n, FFT_THREADS, M.smz[1], s>>>(D.zf, D.mz[1].map);
+    if (D.my[0].n > 0) k_fft_y_multi<R><<<D.my[0].n, FFT_THREADS, M.smy[0], s>>>(D.yf, D.my[0].map);
+    if (D.my[1].n > 0) k_fftr_y_multi<R, false><<<D.my[1].n, FFT_THREADS, M.smy[1], s>>>(D.yf, D.my[1].map);
+    if (D.mx[0].n > 0) {
+        if (energy) k_fft_x_conv_multi<R, true><<<D.mx[0].n, FFT_THREADS, M.smx[0], s>>>(D.x, D.mx[0].map);
+        else k_fft_x_conv_multi<R, false><<<D.mx[0].n, FFT_THREADS, M.smx[0], s>>>(D.x, D.mx[0].map);
     }
-    if (D.my.n > 0) k_fft_y_multi<R><<<D.my.n, FFT_THREADS, M.smy, s>>>(D.yi, D.my.map);
-    if (D.mz.n > 0) k_fft_z_c2r_multi<R><<<D.mz.n, FFT_THREADS, M.smz, s>>>(D.zi, D.mz.map);
+    if (D.mx[1].n > 0) {
+        if (energy) k_fftr_x_conv_multi<R, true><<<D.mx[1].n, FFT_THREADS, M.smx[1], s>>>(D.x, D.mx[1].map);
+        else k_fftr_x_conv_multi<R, false><<<D.mx[1].n, FFT_THREADS, M.smx[1], s>>>(D.x, D.mx[1].map);
+    }
+    if (D.my[0].n > 0) k_fft_y_multi<R><<<D.my[0].n, FFT_THREADS, M.smy[0], s>>>(D.yi, D.my[0].map);
+    if (D.my[1].n > 0) k_fftr_y_multi<R, true><<<D.my[1].n, FFT_THREADS, M.smy[1], s>>>(D.yi, D.my[1].map);
+    if (D.mz[0].n > 0) k_fft_z_c2r_multi<R><<<D.mz[0].n, FFT_THREADS, M.smz[0], s>>>(D.zi, D.mz[0].map);
+    if (D.mz[1].n > 0) k_fftr_z_c2r_multi<R><<<D.mz[1].n, FFT_THREADS, M.smz[1], s>>>(D.zi, D.mz[1].map);
     MDF_CUDA_TRY(cudaGetLastError());
 }
 
@@ -1349,21 +1452,18 @@ static void run_pme_slab(Ctx& c, bool energy)
     F.x.gy = ny;
     F.x.infl += (long long)r * K1p * Kc * K0;
     F.x.my += (long long)r * K1p;
-    k_fft_z_r2c<R><<<grid_of(F.zf), FFT_THREADS, F.smz, c.stream>>>(F.zf);
-    k_fft_y<R><<<grid_of(F.yf), FFT_THREADS, F.smy, c.stream>>>(F.yf);
+    launch_z_r2c(F.zf, F.smz, c.stream);
+    launch_y(F.yf, F.smy, c.stream);
     const int nb = (int)std::min<long long>(148 * 8, ((long long)P * blk + th - 1) / th);
     k_slab_to_blocks<C><<<nb, th, 0, c.stream>>>(slab, sendb, P, K0p, K1, K1p, Kc);
     MDF_CUDA_TRY(cudaGetLastError());
     coll_check(c.coll_a2a(sendb, recvb, (int64_t)(sizeof(C) * blk), (void*)c.stream, c.coll_user), "all-to-all");
-    if (ny > 0) {
-        if (energy) k_fft_x_conv<R, true><<<grid_of(F.x), FFT_THREADS, F.smx, c.stream>>>(F.x);
-        else k_fft_x_conv<R, false><<<grid_of(F.x), FFT_THREADS, F.smx, c.stream>>>(F.x);
-    }
+    if (ny > 0) launch_x_conv(F.x, energy, F.smx, c.stream);
     // back: the x-pass layout [s][x][yl][kc] is already one block per rank
     coll_check(c.coll_a2a(recvb, sendb, (int64_t)(sizeof(C) * blk), (void*)c.stream, c.coll_user), "all-to-all");
     k_blocks_to_slab<C><<<nb, th, 0, c.stream>>>(sendb, slab, K0p, K1, K1p, Kc);
-    k_fft_y<R><<<grid_of(F.yi), FFT_THREADS, F.smy, c.stream>>>(F.yi);
-    k_fft_z_c2r<R><<<grid_of(F.zi), FFT_THREADS, F.smz, c.stream>>>(F.zi);
+    launch_y(F.yi, F.smy, c.stream);
+    launch_z_c2r(F.zi, F.smz, c.stream);
     MDF_CUDA_TRY(cudaGetLastError());
     if (halo) {
         // the potential of my slab in place, and of my window's other planes from their owners
@@ -1592,11 +1692,11 @@ static void run_pme_adjoint(Ctx& c, double gE)
     F.yf.cgrid = F.yi.cgrid = F.x.cgrid = F.zf.cgrid;
     F.yf.gy = F.yi.gy = 2 * K0;
     F.x.gy = 2 * K1;
-    k_fft_z_r2c<R><<<grid_of(F.zf), FFT_THREADS, F.smz, c.stream>>>(F.zf);
-    k_fft_y<R><<<grid_of(F.yf), FFT_THREADS, F.smy, c.stream>>>(F.yf);
-    k_fft_x_conv<R, false><<<grid_of(F.x), FFT_THREADS, F.smx, c.stream>>>(F.x);
-    k_fft_y<R><<<grid_of(F.yi), FFT_THREADS, F.smy, c.stream>>>(F.yi);
-    k_fft_z_c2r<R><<<grid_of(F.zi), FFT_THREADS, F.smz, c.stream>>>(F.zi);
+    launch_z_r2c(F.zf, F.smz, c.stream);
+    launch_y(F.yf, F.smy, c.stream);
+    launch_x_conv(F.x, false, F.smx, c.stream);
+    launch_y(F.yi, F.smy, c.stream);
+    launch_z_c2r(F.zi, F.smz, c.stream);
     k_adj_gather<R><<<grid_blocks(c.n_slots, th), th, 0, c.stream>>>(c.n_slots, c.slot_atom.p, c.xyz.p, B.g, rg, ntot,
                                                                       vs, gE, c.adj_dq_slot.p, c.status.p);
     MDF_CUDA_TRY(cudaGetLastError());
