@@ -247,6 +247,7 @@ __device__ __forceinline__ void fft_z_c2r_dev(const FFTZArgs<R>& A, int bx, int 
             A = cconj(A);
             B = cconj(B);
         }
+        if (k == 0 || 2 * k == K2) A.y = B.y = 0;   // real line: see regs_z_c2r_dev
         const C Z = {A.x - B.y, A.y + B.x};
         bufA[line * K2 + k] = Z;
     }
