@@ -39,6 +39,11 @@ __device__ __forceinline__ C cmul(C a, C b)
     return r;
 }
 
+// Rounded product, never contracted with an addition: the convolution gives the
+// same bits with energies (through shared memory) and without (in registers).
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
 template <typename C>
 __device__ __forceinline__ C cconj(C a)
 {
@@ -460,8 +465,8 @@ __device__ __forceinline__ void regs_x_conv_dev(const FFTXArgs<R>& A, int bx, in
 #pragma unroll
             for (int k = 0; k < N; ++k) {
                 const R c = l < live ? fl[(long long)(j + k * nb) * Kc + l] : (R)0;
-                v[k].x *= c;
-                v[k].y *= c;
+                v[k].x = mul_rn(v[k].x, c);
+                v[k].y = mul_rn(v[k].y, c);
             }
             RDft<N, true, R, C>::run(v);   // first stage of the inverse with the radices reversed
             C* o = turn + j * N * M.si + l * M.sl;
