@@ -422,28 +422,16 @@ void eval_async_impl(Ctx& c, uint32_t flags)
         c.need_clear = false;
     }
     // The exclusion, 1-4, bonded and PME kernels only read positions and
-    // charges and add into the fixed-point accumulators, so they run on the
-    // side stream while the main stream packs, prunes and runs the pair
+    // charges and add into the fixed-point accumulators, so they run on two
+    // side streams while the main stream packs, prunes and runs the pair
     // kernel; the main stream waits for them before k_finalize.  With timing enabled every
     // kernel runs on the main stream so the per-phase times are separable.
     const bool want_pme = phys || (flags & MDF_COMPUTE_PME_REFERENCE);
     const bool overlap = want_pme && !c.timing;
-    if (overlap) {
-        MDF_CUDA_TRY(cudaEventRecord(c.ev_fork, s));
-        MDF_CUDA_TRY(cudaStreamWaitEvent(c.side, c.ev_fork, 0));
-        c.stream = c.side;
-        try {
-            launch_exclusions(c, energy);
-            launch_bonded(c, energy);
-            launch_pme(c, energy);
-        } catch (...) {
-            c.stream = s;
-            throw;
-        }
-        c.stream = s;
-        c.have_pme_ref = !phys;
-        MDF_CUDA_TRY(cudaEventRecord(c.ev_join, c.side));
-    }
+    if (overlap) MDF_CUDA_TRY(cudaEventRecord(c.ev_fork, s));
+    // the main stream's kernels go first: the pair kernel ends the evaluation of
+    // all but small systems, and the host's launches of the side streams would
+    // hold its chain back (the side stream's priority places its blocks anyway)
     pack_positions(c);
     mark(c, "pack");
     if (c.p.prune_every > 0) {
@@ -459,17 +447,34 @@ void eval_async_impl(Ctx& c, uint32_t flags)
     }
     launch_nonbonded(c, energy);
     mark(c, "pairs");
-    if (!overlap) {
-        launch_exclusions(c, energy);
-        mark(c, "excl_14");
-        launch_bonded(c, energy);
-        mark(c, "bonded");
-    }
-    if (want_pme && !overlap) {
-        launch_pme(c, energy);
+    if (overlap) {
+        try {
+            MDF_CUDA_TRY(cudaStreamWaitEvent(c.side, c.ev_fork, 0));
+            c.stream = c.side;
+            launch_pme(c, energy);
+            MDF_CUDA_TRY(cudaEventRecord(c.ev_join, c.side));
+            MDF_CUDA_TRY(cudaStreamWaitEvent(c.side2, c.ev_fork, 0));
+            c.stream = c.side2;
+            launch_terms(c, energy, true, true);
+            MDF_CUDA_TRY(cudaEventRecord(c.ev_join2, c.side2));
+        } catch (...) {
+            c.stream = s;
+            throw;
+        }
+        c.stream = s;
         c.have_pme_ref = !phys;
+        MDF_CUDA_TRY(cudaStreamWaitEvent(s, c.ev_join, 0));
+        MDF_CUDA_TRY(cudaStreamWaitEvent(s, c.ev_join2, 0));
+    } else {
+        launch_terms(c, energy, false, true);
+        mark(c, "excl_14");
+        launch_terms(c, energy, true, false);
+        mark(c, "bonded");
+        if (want_pme) {
+            launch_pme(c, energy);
+            c.have_pme_ref = !phys;
+        }
     }
-    if (overlap) MDF_CUDA_TRY(cudaStreamWaitEvent(s, c.ev_join, 0));
     if (slab_mode(c)) {
         // energies, virial and pair count summed; the forces by reduce-scatter
         // of the accumulators and all-gather of the finished forces
@@ -751,16 +756,18 @@ int mdf_create(const mdf_topology* top, const mdf_params* p, mdf_ctx** out)
         MDF_CUDA_TRY(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
         c.own_stream = true;
         {
-            // The side stream (exclusions, 1-4, bonded, PME) gets the highest
+            // The side streams (PME; exclusions, 1-4, bonded) get the highest
             // priority: its kernels are short and few-block, and scheduled
             // first they finish inside the pair kernel instead of stretching
             // its tail (c1 mixed: 0.364 vs 0.386 ms per evaluation).
             int lo = 0, hi = 0;
             MDF_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));
             MDF_CUDA_TRY(cudaStreamCreateWithPriority(&c.side, cudaStreamNonBlocking, hi));
+            MDF_CUDA_TRY(cudaStreamCreateWithPriority(&c.side2, cudaStreamNonBlocking, hi));
         }
         MDF_CUDA_TRY(cudaEventCreateWithFlags(&c.ev_fork, cudaEventDisableTiming));
         MDF_CUDA_TRY(cudaEventCreateWithFlags(&c.ev_join, cudaEventDisableTiming));
+        MDF_CUDA_TRY(cudaEventCreateWithFlags(&c.ev_join2, cudaEventDisableTiming));
         MDF_CUDA_TRY(cudaHostAlloc((void**)&c.h_scal, sizeof(unsigned long long) * NUM_SCAL, cudaHostAllocMapped));
         memset(c.h_scal, 0, sizeof(unsigned long long) * NUM_SCAL);
         MDF_CUDA_TRY(cudaHostGetDevicePointer((void**)&c.d_hscal, c.h_scal, 0));
@@ -844,8 +851,10 @@ void mdf_destroy(mdf_ctx* ctx)
     c.md_v.release(); c.md_invm.release(); c.md_xref.release(); c.min_x.release(); c.min_f.release(); c.md_words.release();
     if (c.stream && c.own_stream) cudaStreamDestroy(c.stream);
     if (c.side) cudaStreamDestroy(c.side);
+    if (c.side2) cudaStreamDestroy(c.side2);
     if (c.ev_fork) cudaEventDestroy(c.ev_fork);
     if (c.ev_join) cudaEventDestroy(c.ev_join);
+    if (c.ev_join2) cudaEventDestroy(c.ev_join2);
     delete ctx;
 }
 

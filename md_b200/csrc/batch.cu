@@ -57,8 +57,9 @@ struct mdf_batch {
     // one launch per kernel for all systems (uniform launch parameters), or
     // every system's own kernel chain in the graph
     bool multi = false;
-    cudaStream_t side = nullptr;         // PME, bonded, exclusions: concurrent with pack/prune/pairs
-    cudaEvent_t ev_fork2 = nullptr, ev_join2 = nullptr;
+    cudaStream_t side = nullptr;         // PME: concurrent with pack/prune/pairs
+    cudaStream_t side2 = nullptr;        // bonded terms, exclusions, 1-4: the same
+    cudaEvent_t ev_fork2 = nullptr, ev_join2 = nullptr, ev_join3 = nullptr;
     // per-kernel argument arrays of the multi form (rebuilt before each capture)
     DevBuf<unsigned char> args;          // one allocation, the arrays below point into it
     size_t args_cap = 0;
@@ -193,9 +194,7 @@ struct MultiArgs {
     std::vector<PruneArgs> prune;
     std::vector<PairF32Args> pf32;
     std::vector<PairF64Args> p64;
-    std::vector<ExclArgs> excl;
-    std::vector<Pair14Args> p14;
-    std::vector<BondedArgs> bonded;
+    std::vector<TermArgs> terms;
     std::vector<ZeroArgs> zero;
     std::vector<SpreadArgs> spread;
     std::vector<FFTZArgs<R>> zf, zi;
@@ -207,7 +206,7 @@ struct MultiArgs {
     // systems (one entry per block actually needed: no idle blocks)
     std::vector<int2> map_pack, map_zero, map_spread, map_z[2], map_y[2], map_x[2], map_gather, map_fin;
     FFTChainMax fm{};
-    int gx_prune = 0, gx_pairs = 0, gx_excl = 0, gx_14 = 0, gx_bonded = 0;
+    int gx_prune = 0, gx_pairs = 0, gx_terms = 0;
     size_t dyn_pairs = 0;
     int threads = 256;
     bool prune_on = false, use_switch = false, energy = false, persist = false, half = false;
@@ -222,9 +221,7 @@ struct MultiDev {
     const PruneArgs* prune;
     const PairF32Args* pf32;
     const PairF64Args* p64;
-    const ExclArgs* excl;
-    const Pair14Args* p14;
-    const BondedArgs* bonded;
+    const TermArgs* terms;
     const ZeroArgs* zero;
     const SpreadArgs* spread;
     FFTChainDev<R> fft;
@@ -291,9 +288,7 @@ MultiDev<R> prepare_multi(mdf_batch* b, uint32_t flags, MultiArgs<R>& M, double*
             M.p64.push_back(make_pair_f64_args(c, &dyn));
             M.dyn_pairs = std::max(M.dyn_pairs, dyn);
         }
-        M.excl.push_back(make_excl_args(c));
-        M.p14.push_back(make_pair14_args(c));
-        M.bonded.push_back(make_bonded_args(c, false, c.f_atom.p, c.acc.p, c.status.p));
+        M.terms.push_back(make_term_args(c, energy, true, true));
         const long long ntot = (long long)c.K[0] * c.K[1] * c.K[2];
         ZeroArgs z;
         z.gx = grid_blocks(ntot, 256 * 8);
@@ -345,9 +340,7 @@ MultiDev<R> prepare_multi(mdf_batch* b, uint32_t flags, MultiArgs<R>& M, double*
     }
     M.gx_prune = gmax(M.prune);
     M.gx_pairs = sizeof(R) == 4 ? gmax(M.pf32) : gmax(M.p64);
-    M.gx_excl = gmax(M.excl);
-    M.gx_14 = gmax(M.p14);
-    M.gx_bonded = gmax(M.bonded);
+    M.gx_terms = gmax(M.terms);
     for (int s = 0; s < n; ++s) {
         add_blocks(M.map_pack, s, M.pack[s].gx, 1);
         add_blocks(M.map_zero, s, M.zero[s].gx, 1);
@@ -357,7 +350,7 @@ MultiDev<R> prepare_multi(mdf_batch* b, uint32_t flags, MultiArgs<R>& M, double*
     }
     // one device allocation for every array
     const size_t total = arr_bytes(M.pack) + arr_bytes(M.prune) + arr_bytes(M.pf32) + arr_bytes(M.p64) +
-                         arr_bytes(M.excl) + arr_bytes(M.p14) + arr_bytes(M.bonded) + arr_bytes(M.zero) +
+                         arr_bytes(M.terms) + arr_bytes(M.zero) +
                          arr_bytes(M.spread) + arr_bytes(M.zf) + arr_bytes(M.yf) + arr_bytes(M.x) +
                          arr_bytes(M.yi) + arr_bytes(M.zi) + arr_bytes(M.gather) + arr_bytes(M.fin) +
                          arr_bytes(M.map_pack) + arr_bytes(M.map_zero) + arr_bytes(M.map_spread) +
@@ -378,9 +371,7 @@ MultiDev<R> prepare_multi(mdf_batch* b, uint32_t flags, MultiArgs<R>& M, double*
     put(M.prune, D.prune);
     put(M.pf32, D.pf32);
     put(M.p64, D.p64);
-    put(M.excl, D.excl);
-    put(M.p14, D.p14);
-    put(M.bonded, D.bonded);
+    put(M.terms, D.terms);
     put(M.zero, D.zero);
     put(M.spread, D.spread);
     put(M.zf, D.fft.zf);
@@ -426,14 +417,14 @@ void enqueue_multi(mdf_batch* b, const MultiArgs<R>& M, const MultiDev<R>& D, co
     k_batch_scatter<<<grid, th, 0, b->main>>>(b->d_off.p, d_pos, b->d_xyz_ptr.p);
     MDF_CUDA_TRY(cudaGetLastError());
     long long k = 2;   // scatter + finalize
-    // side stream: exclusions, 1-4, bonded terms, PME (they only read positions
-    // and charges and add into the fixed-point accumulators)
+    // side streams: PME, and the exclusions, 1-4 and bonded terms (they only
+    // read positions and charges and add into the fixed-point accumulators)
     MDF_CUDA_TRY(cudaEventRecord(b->ev_fork2, b->main));
     MDF_CUDA_TRY(cudaStreamWaitEvent(b->side, b->ev_fork2, 0));
-    launch_exclusions_multi(D.excl, M.gx_excl, D.p14, M.gx_14, n, M.energy, b->side);
-    k += (M.gx_excl > 0) + (M.gx_14 > 0);
-    launch_bonded_multi(D.bonded, n, M.gx_bonded, M.energy, b->side);
-    k += M.gx_bonded > 0;
+    MDF_CUDA_TRY(cudaStreamWaitEvent(b->side2, b->ev_fork2, 0));
+    launch_terms_multi(D.terms, n, M.gx_terms, M.energy, b->side2);
+    k += M.gx_terms > 0;
+    MDF_CUDA_TRY(cudaEventRecord(b->ev_join3, b->side2));
     launch_pme_multi<R>(D.zero, D.zero_m, D.spread, D.spread_m, D.fft, M.fm, D.gather, D.gather_m, M.energy,
                         b->side);
     k += 3;   // grid clear, spread, gather
@@ -462,6 +453,7 @@ void enqueue_multi(mdf_batch* b, const MultiArgs<R>& M, const MultiDev<R>& D, co
         ++k;
     }
     MDF_CUDA_TRY(cudaStreamWaitEvent(b->main, b->ev_join2, 0));
+    MDF_CUDA_TRY(cudaStreamWaitEvent(b->main, b->ev_join3, 0));
     launch_finalize_multi(D.fin, D.fin_m, b->main);
     if (copies)
         MDF_CUDA_TRY(cudaMemcpyAsync(b->h_forces, b->d_forces.p, sizeof(double) * b->total, cudaMemcpyDeviceToHost,
@@ -667,9 +659,11 @@ int mdf_batch_create(int nsys, const mdf_topology* const* topos, const mdf_param
             int lo = 0, hi = 0;   // the short PME / bonded kernels first (as in one context)
             MDF_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));
             MDF_CUDA_TRY(cudaStreamCreateWithPriority(&b->side, cudaStreamNonBlocking, hi));
+            MDF_CUDA_TRY(cudaStreamCreateWithPriority(&b->side2, cudaStreamNonBlocking, hi));
         }
         MDF_CUDA_TRY(cudaEventCreateWithFlags(&b->ev_fork2, cudaEventDisableTiming));
         MDF_CUDA_TRY(cudaEventCreateWithFlags(&b->ev_join2, cudaEventDisableTiming));
+        MDF_CUDA_TRY(cudaEventCreateWithFlags(&b->ev_join3, cudaEventDisableTiming));
         b->join.assign(nsys, nullptr);
         for (int s = 0; s < nsys; ++s) MDF_CUDA_TRY(cudaEventCreateWithFlags(&b->join[s], cudaEventDisableTiming));
         MDF_CUDA_TRY(cudaHostAlloc((void**)&b->h_pos, sizeof(double) * b->total, cudaHostAllocDefault));
@@ -719,7 +713,9 @@ void mdf_batch_destroy(mdf_batch* b)
     if (b->fork) cudaEventDestroy(b->fork);
     if (b->ev_fork2) cudaEventDestroy(b->ev_fork2);
     if (b->ev_join2) cudaEventDestroy(b->ev_join2);
+    if (b->ev_join3) cudaEventDestroy(b->ev_join3);
     if (b->side) cudaStreamDestroy(b->side);
+    if (b->side2) cudaStreamDestroy(b->side2);
     b->args.release();
     for (auto& S : b->stage) {
         if (S.h_scal) cudaFreeHost(S.h_scal);

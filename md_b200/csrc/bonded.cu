@@ -13,6 +13,7 @@
 #include "kargs.cuh"
 #include "mdf_device.cuh"
 #include "mdf_internal.cuh"
+#include "pair_terms.cuh"
 
 namespace mdf {
 
@@ -124,15 +125,15 @@ __device__ void cmap_eval(const double* __restrict__ coeff, int res, int set, do
 }
 
 template <bool PHYS, bool ENERGY>
-__device__ __forceinline__ void bonded_dev(const BondedArgs& A)
+__device__ __forceinline__ void bonded_dev(const BondedArgs& A, int bx)
 {
     unsigned long long* __restrict__ f = A.f;
     unsigned long long* __restrict__ acc = A.acc;
     unsigned* st = A.st;
     const double PI = 3.14159265358979323846;
     int seg = 0;
-    while (seg < 5 && (int)blockIdx.x >= A.blk0[seg + 1]) ++seg;
-    int i = A.lo[seg] + ((int)blockIdx.x - A.blk0[seg]) * blockDim.x + threadIdx.x;
+    while (seg < 5 && bx >= A.blk0[seg + 1]) ++seg;
+    int i = A.lo[seg] + (bx - A.blk0[seg]) * blockDim.x + threadIdx.x;
     const double* x = A.xyz;
     double e = 0.0;
     int eidx = MDF_E_BOND;
@@ -267,18 +268,43 @@ __device__ __forceinline__ void bonded_dev(const BondedArgs& A)
     }
 }
 
+// All the FP64 terms of listed atoms in one launch: bonded terms, then excluded
+// pairs, then 1-4 pairs, each in blocks of its own.  What bounds them is latency
+// (a few gathers and double-precision functions per thread), so side by side
+// they take the time of the longest instead of the sum of three launches, and
+// on a stream of their own they no longer stand before the PME chain, which
+// ends the evaluation of small systems (evaluations back to back: 2,780 atoms
+// 75 -> 60 us, 28k 128 -> 106, 100k 274 and 100k FP64 529 either way).
 template <bool PHYS, bool ENERGY>
-__global__ void __launch_bounds__(256) k_bonded(BondedArgs A)
+__device__ __forceinline__ void terms_dev(const TermArgs& A)
 {
-    bonded_dev<PHYS, ENERGY>(A);
+    constexpr int SEM = PHYS ? MDF_SEM_PHYSICAL : MDF_SEM_REFERENCE;
+    int bx = (int)blockIdx.x;
+    if (bx < A.b.gx) {
+        bonded_dev<PHYS, ENERGY>(A.b, bx);
+        return;
+    }
+    bx -= A.b.gx;
+    if (bx < A.e.gx) {
+        exclusions_dev<SEM, ENERGY>(A.e, bx);
+        return;
+    }
+    bx -= A.e.gx;
+    if (bx < A.p.gx) pairs14_dev<SEM, ENERGY>(A.p, bx);
 }
 
 template <bool PHYS, bool ENERGY>
-__global__ void __launch_bounds__(256) k_bonded_multi(const BondedArgs* __restrict__ As)
+__global__ void __launch_bounds__(256) k_terms(const __grid_constant__ TermArgs A)
 {
-    const BondedArgs& A = As[blockIdx.z];
+    terms_dev<PHYS, ENERGY>(A);
+}
+
+template <bool PHYS, bool ENERGY>
+__global__ void __launch_bounds__(256) k_terms_multi(const TermArgs* __restrict__ As)
+{
+    const TermArgs& A = As[blockIdx.z];
     if ((int)blockIdx.x >= A.gx) return;
-    bonded_dev<PHYS, ENERGY>(A);
+    terms_dev<PHYS, ENERGY>(A);
 }
 
 // The six term lists in one launch: this rank's share of each (all of them
@@ -311,38 +337,58 @@ BondedArgs make_bonded_args(const Ctx& c, bool whole, unsigned long long* f, uns
     return A;
 }
 
-static void launch_bonded_args(const Ctx& c, const BondedArgs& A, bool energy)
+// This rank's terms: the bonded lists and/or the excluded and 1-4 pairs.
+TermArgs make_term_args(const Ctx& c, bool energy, bool bonded, bool pairs)
+{
+    TermArgs A;
+    A.b = make_bonded_args(c, false, c.f_atom.p, c.acc.p, c.status.p);
+    A.e = make_excl_args(c);
+    A.p = make_pair14_args(c);
+    if (!bonded) A.b.gx = 0;
+    // REFERENCE excluded pairs have an energy and no force
+    if (!pairs || A.e.n == 0 || (c.p.semantics != MDF_SEM_PHYSICAL && !energy)) A.e.gx = 0;
+    if (!pairs || A.p.n == 0) A.p.gx = 0;
+    A.gx = A.b.gx + A.e.gx + A.p.gx;
+    A.gy = 1;
+    return A;
+}
+
+static void launch_term_args(const Ctx& c, const TermArgs& A, bool energy)
 {
     if (A.gx == 0) return;
     const int th = 256;
     if (c.p.semantics == MDF_SEM_PHYSICAL) {
-        if (energy) k_bonded<true, true><<<grid_of(A), th, 0, c.stream>>>(A);
-        else k_bonded<true, false><<<grid_of(A), th, 0, c.stream>>>(A);
+        if (energy) k_terms<true, true><<<grid_of(A), th, 0, c.stream>>>(A);
+        else k_terms<true, false><<<grid_of(A), th, 0, c.stream>>>(A);
     } else {
-        if (energy) k_bonded<false, true><<<grid_of(A), th, 0, c.stream>>>(A);
-        else k_bonded<false, false><<<grid_of(A), th, 0, c.stream>>>(A);
+        if (energy) k_terms<false, true><<<grid_of(A), th, 0, c.stream>>>(A);
+        else k_terms<false, false><<<grid_of(A), th, 0, c.stream>>>(A);
     }
     MDF_CUDA_TRY(cudaGetLastError());
 }
 
-void launch_bonded(Ctx& c, bool energy)
+void launch_terms(Ctx& c, bool energy, bool bonded, bool pairs)
 {
-    const BondedArgs A = make_bonded_args(c, false, c.f_atom.p, c.acc.p, c.status.p);
+    const TermArgs A = make_term_args(c, energy, bonded, pairs);
     if (A.gx == 0) return;
-    launch_bonded_args(c, A, energy);
+    launch_term_args(c, A, energy);
     c.launches += 1;
 }
 
 void launch_bonded_into(Ctx& c, bool energy, unsigned long long* f, unsigned long long* acc, unsigned* st)
 {
-    launch_bonded_args(c, make_bonded_args(c, true, f, acc, st), energy);
+    TermArgs A{};
+    A.b = make_bonded_args(c, true, f, acc, st);
+    A.gx = A.b.gx;
+    A.gy = 1;
+    launch_term_args(c, A, energy);
 }
 
-void launch_bonded_multi(const BondedArgs* d_args, int nsys, int gx, bool energy, cudaStream_t s)
+void launch_terms_multi(const TermArgs* d_args, int nsys, int gx, bool energy, cudaStream_t s)
 {
     if (gx == 0) return;
-    if (energy) k_bonded_multi<true, true><<<dim3(gx, 1, nsys), 256, 0, s>>>(d_args);
-    else k_bonded_multi<true, false><<<dim3(gx, 1, nsys), 256, 0, s>>>(d_args);
+    if (energy) k_terms_multi<true, true><<<dim3(gx, 1, nsys), 256, 0, s>>>(d_args);
+    else k_terms_multi<true, false><<<dim3(gx, 1, nsys), 256, 0, s>>>(d_args);
     MDF_CUDA_TRY(cudaGetLastError());
 }
 

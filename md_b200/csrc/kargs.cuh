@@ -252,6 +252,15 @@ struct BondedArgs {
     unsigned* st;
 };
 
+// Bonded terms, excluded pairs and 1-4 pairs of one system (gx = the sum of
+// their blocks; a part left out has gx = 0).
+struct TermArgs {
+    int gx, gy;
+    BondedArgs b;
+    ExclArgs e;
+    Pair14Args p;
+};
+
 // --------------------------------------------------------------------- PME
 struct GridGeom {
     int K[3];
@@ -413,10 +422,9 @@ inline void set_pair_split(PairF32Args& a, int split, int warps_per_block)
 }
 ExclArgs make_excl_args(const Ctx& c);
 Pair14Args make_pair14_args(const Ctx& c);
-void launch_exclusions_multi(const ExclArgs* d_excl, int gx_excl, const Pair14Args* d_14, int gx_14, int nsys,
-                             bool energy, cudaStream_t s);
 BondedArgs make_bonded_args(const Ctx& c, bool whole, unsigned long long* f, unsigned long long* acc, unsigned* st);
-void launch_bonded_multi(const BondedArgs* d_args, int nsys, int gx, bool energy, cudaStream_t s);
+TermArgs make_term_args(const Ctx& c, bool energy, bool bonded, bool pairs);
+void launch_terms_multi(const TermArgs* d_args, int nsys, int gx, bool energy, cudaStream_t s);
 template <typename R> FFTChain<R> make_fft_chain(const Ctx& c, bool energy);
 SpreadArgs make_spread_args(const Ctx& c);
 template <typename R> GatherArgs<R> make_gather_args(const Ctx& c);

@@ -120,7 +120,8 @@ struct Ctx {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaStream_t side = nullptr;         // the PME chain runs here, concurrently with the pair kernel
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaStream_t side2 = nullptr;        // the listed FP64 terms run here
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr;
     mdf_params p{};
     int N = 0;
     int ntypes = 0;
@@ -352,8 +353,7 @@ inline bool half_layout(const Ctx& c) { return c.p.pair_layout == 1 && c.p.prune
 // since the last prune (one context per system; with several ranks it prunes every evaluation)
 inline bool self_pruning(const Ctx& c) { return c.p.prune_every < 0 && c.p.nranks <= 1 && c.xq_snap.p != nullptr; }
 void launch_nonbonded(Ctx& c, bool energy);
-void launch_exclusions(Ctx& c, bool energy);
-void launch_bonded(Ctx& c, bool energy);
+void launch_terms(Ctx& c, bool energy, bool bonded, bool pairs);
 void launch_bonded_into(Ctx& c, bool energy, unsigned long long* f, unsigned long long* acc, unsigned* st);
 void setup_pme(Ctx& c);
 void launch_pme(Ctx& c, bool energy);
