@@ -155,8 +155,8 @@ typedef struct {
     double prune_margin;
     /* Launch shapes (results do not depend on them; mdf_batch_autotune picks
      * them): warps per block of the pair kernel (2, 4 or 8; 0 = 8) and FFT
-     * lines per block (1, 2, 4, 8, 16 or 32; 0 = chosen per grid size: 4 for
-     * 100 or 216 points, 16 for 32, so small grids keep every thread busy). */
+     * lines per block (1, 2, 4, 8, 16 or 32; 0 = chosen per grid size,
+     * so that small grids keep every thread busy). */
     int32_t pair_warps;
     int32_t fft_lines;
     /* Work split over nranks contexts (one per GPU, PHYSICAL semantics; 0 or
