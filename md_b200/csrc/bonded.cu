@@ -271,7 +271,8 @@ __device__ __forceinline__ void bonded_dev(const BondedArgs& A, int bx)
 // All the FP64 terms of listed atoms in one launch: bonded terms, then excluded
 // pairs, then 1-4 pairs, each in blocks of its own.  What bounds them is latency
 // (a few gathers and double-precision functions per thread), so side by side
-// they take the time of the longest instead of the sum of three launches, and
+// they take the time of the longest instead of the sum of three launches (100k
+// atoms 26 -> 15 us), and
 // on a stream of their own they no longer stand before the PME chain, which
 // ends the evaluation of small systems (evaluations back to back: 2,780 atoms
 // 75 -> 60 us, 28k 128 -> 106, 100k 274 and 100k FP64 529 either way).
