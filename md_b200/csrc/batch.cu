@@ -211,6 +211,7 @@ struct MultiArgs {
     int threads = 256;
     bool prune_on = false, use_switch = false, energy = false, persist = false, half = false;
     int prune_warps = 1;
+    bool prune_wide = false;
     bool parts = false;    // some system's lists are cut into parts
     bool lj_smem = true;   // every system's LJ table in shared memory (one kernel form for the batch)
 };
@@ -279,6 +280,7 @@ MultiDev<R> prepare_multi(mdf_batch* b, uint32_t flags, MultiArgs<R>& M, double*
         }
         M.pack.push_back(make_pack_args<R>(c));
         M.prune.push_back(make_prune_args(c, M.half));
+        M.prune_wide = M.prune_wide || prune_wide_clusters(c);
         if (sizeof(R) == 4) {
             size_t dyn = 0;
             M.pf32.push_back(make_pair_f32_args(c, &dyn));
@@ -435,7 +437,8 @@ void enqueue_multi(mdf_batch* b, const MultiArgs<R>& M, const MultiDev<R>& D, co
     launch_pack_multi<R>(D.pack, D.pack_m, b->main);
     ++k;
     if (M.prune_on) {
-        launch_prune_multi(D.prune, n, M.gx_prune, M.prune_warps, M.half, self_pruning(b->sys[0]->c), b->main);
+        launch_prune_multi(D.prune, n, M.gx_prune, M.prune_warps, M.half, M.prune_wide, self_pruning(b->sys[0]->c),
+                           b->main);
         ++k;
     }
     if (M.gx_pairs > 0) {

@@ -53,7 +53,7 @@ struct PruneArgs {
     const ILRange* ilist;
     const PairEntry* plist;
     const float4* xf;
-    const double4* xd;      // FP64 offsets (snap_d only)
+    const double4* xd;      // FP64 contexts: the offsets in FP64 (snap_d, wide clusters)
     const float4 *centerf, *box;
     int box_fine;           // box padding small enough for the acceptance by boxes
     ShiftTable shifts;
@@ -404,7 +404,8 @@ template <typename R> void launch_pack_multi(const PackArgs<R>* d_args, BlockMap
 PruneArgs make_prune_args(const Ctx& c, bool half);
 void set_prune_warps(PruneArgs& A, long long ncl);   // by the clusters of the whole launch
 void ensure_half_lists(Ctx& c);
-void launch_prune_multi(const PruneArgs* d_args, int nsys, int gx, int warps, bool half, bool selfp, cudaStream_t s);
+void launch_prune_multi(const PruneArgs* d_args, int nsys, int gx, int warps, bool half, bool wide, bool selfp,
+                        cudaStream_t s);
 PairF32Args make_pair_f32_args(const Ctx& c, size_t* dyn);
 void launch_pairs_f32_multi(const PairF32Args* d_args, int nsys, int gx, int threads, size_t dyn, bool energy,
                             bool use_switch, bool persist, bool half, bool lj_smem, bool parts, cudaStream_t s);

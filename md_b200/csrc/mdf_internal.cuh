@@ -169,6 +169,7 @@ struct Ctx {
     int ncol_x = 0, ncol_y = 0, ncols = 0;
     int n_clusters = 0, n_slots = 0;
     bool have_list = false;
+    bool wide_clusters = false;    // some cluster of the list is wider than the FP32 prune test is meant for
     DevBuf<int2> atom_col;          // [N]
     DevBuf<int> col_count, col_start, col_cstart;   // [ncols + 1]
     DevBuf<int> col_atoms;         // [N] atoms bucketed by column
@@ -194,8 +195,8 @@ struct Ctx {
     DevBuf<unsigned char> xq_snap; // self-pruning mode: the cluster-frame positions of the last prune, per slot
     int since_prune = 0;
     bool pruned_valid = false;
-    DevBuf<int> d_build;           // [4] list entries claimed by the search
-    int* h_build = nullptr;        // pinned: cluster count, entry count, status of the last build
+    DevBuf<int> d_build;           // [4] list entries claimed by the search, wide clusters seen
+    int* h_build = nullptr;        // pinned: cluster count, entry count, wide clusters, status of the last build
 
     // accumulators.  The force accumulators are cleared by the kernel that
     // reads them (k_finalize); the scalar block is copied to the host and then
@@ -347,6 +348,8 @@ void build_pairlist(Ctx& c);
 void build_bands(Ctx& c);   // rank bands and halo plane lists of a split evaluation
 void pack_positions(Ctx& c);
 void prune_pairlist(Ctx& c, bool whole_entries = false);
+// the prune tests wide clusters in FP64
+inline bool prune_wide_clusters(const Ctx& c) { return c.wide_clusters && c.p.precision != MDF_PREC_MIXED; }
 // half-entry lists in use by the pair kernel (layout 1, pruned)
 inline bool half_layout(const Ctx& c) { return c.p.pair_layout == 1 && c.p.prune_every != 0; }
 // prune_every < 0: the device prunes when an atom moved more than prune_margin / 2

@@ -400,6 +400,11 @@ __device__ __forceinline__ bool excluded_entry(int I, int la, int a, int b, cons
     return true;
 }
 
+// Clusters beyond this extent (A) are pruned by the WIDE form in FP64 contexts;
+// below it, whatever the atoms move until the next build, the FP32 test's
+// rounding stays near 1e-2 A^2.  Liquids stay at 5 to 10 A.
+constexpr float WIDE_EXTENT = 64.f;
+
 constexpr int SEARCH_WARPS = 4;
 constexpr int SEARCH_CAP = 512;   // entries a warp buffers (~125 per i cluster at liquid density, 10 + 2 A)
 
@@ -440,6 +445,7 @@ __global__ void __launch_bounds__(32 * SEARCH_WARPS) k_pair_search(
     const int col = cluster_col[I];
     const int cx = col / g.ncy, cy = col % g.ncy;
     const float4 lo = bb_lo[I], hi = bb_hi[I];
+    if (lane == 0 && fmaxf(hi.x - lo.x, fmaxf(hi.y - lo.y, hi.z - lo.z)) > WIDE_EXTENT) d_total[1] = 1;
     const int nvi = (int)lo.w;
     const int nxc = 2 * g.Rx + 1, ncand = nxc * (2 * g.Ry + 1);
     const float Lx = (float)g.L[0], Ly = (float)g.L[1], Lz = (float)g.L[2];
@@ -593,9 +599,13 @@ __global__ void __launch_bounds__(32 * SEARCH_WARPS) k_pair_search(
 // from the i cluster's start offset in the outer list.  The test ignores the
 // entry's exclusion mask (an entry whose only close pairs are excluded is
 // kept; the pair kernel applies the mask), so it keeps a superset of the exact
-// set, and it runs in FP32 in both precisions: the frame offsets are exact to
-// ~1e-6 A and |a - b|^2 = |a|^2 + |b|^2 - 2 a.b rounds by ~1e-4 A^2, far
-// inside the radius' 0.02 A margin.
+// set, and it runs in FP32 in both precisions: |a - b|^2 = |a|^2 + |b|^2 - 2 a.b
+// rounds with the square of the clusters' extents, by ~1e-4 A^2 at liquid
+// density and ~2e-3 A^2 at half extents of 16 A (BoxF.fine), inside the radius'
+// 0.02 A margin (0.1 A^2 at a cutoff of 3 A).  Wider clusters, those of very
+// dilute systems, lose pairs near the cutoff from extents of some hundred A on:
+// FP64 contexts that have them test their entries in FP64 (WIDE, prune_wide),
+// mixed contexts don't.
 //
 // W warps share an i cluster (32 entries each per round).  An entry is first
 // tested lane by lane through the clusters' current boxes (k_pack): farther
@@ -636,12 +646,31 @@ __device__ __forceinline__ float min_with2(float m, F32x2 v)   // min(m, v.lo, v
 
 constexpr int PRUNE_WARPS = 8;   // largest block
 
+// One entry in FP64, without the expansion: bit h set when half h of the i
+// cluster has an atom pair within the radius.  Called for clusters too wide for
+// the FP32 test; not inlined, so that it takes no registers from it.
+__device__ __noinline__ unsigned prune_wide(const double4* __restrict__ xi, const double4* __restrict__ xj, float ox,
+                                            float oy, float oz, float rc2)
+{
+    unsigned near = 0;
+    for (int j = 0; j < CLUSTER && near != 3u; ++j) {
+        const double4 b = xj[j];
+        const double qx = b.x + ox, qy = b.y + oy, qz = b.z + oz;
+        for (int i = 0; i < CLUSTER; ++i) {
+            const double4 a = xi[i];
+            const double dx = a.x - qx, dy = a.y - qy, dz = a.z - qz;
+            if (fma(dx, dx, fma(dy, dy, dz * dz)) < rc2) near |= 1u << (i / 4);
+        }
+    }
+    return near;
+}
+
 // HALF: the half layout (4 x 8).  Each half of the i cluster (atoms 0-3, 4-7)
 // is tested on its own and an entry goes to the list of every half that has an
 // atom pair within the radius.  The outer range [start, start + count) of i
 // cluster I owns the slots [2 start + h count, 2 start + (h + 1) count) of the
 // half list; item 2 w + h of this launch describes half h (ILRange.pad = h).
-template <int W, bool HALF>
+template <int W, bool HALF, bool WIDE>
 __device__ __forceinline__ void prune_dev(const PruneArgs& A)
 {
     // self-pruning: the list pruned last time still holds every pair within the cutoff
@@ -700,6 +729,15 @@ __device__ __forceinline__ void prune_dev(const PruneArgs& A)
             const float far2 = fminf(ux * ux + wy + wz, fminf(wx + uy * uy + wz, wx + wy + uz * uz));
             k0 = todo && far2 < rc2 && A.box_fine && bi.fine && bj.fine;
             todo = todo && !k0;
+        }
+        if (WIDE && todo && !(bi.fine && bj.fine)) {
+            const float4 cJ = A.centerf[my.j];
+            const unsigned near = prune_wide(A.xd + (size_t)I * CLUSTER, A.xd + (size_t)my.j * CLUSTER,
+                                             -(((cI.x - cJ.x) - s6[0]) - s6[3]), -(((cI.y - cJ.y) - s6[1]) - s6[4]),
+                                             -(((cI.z - cJ.z) - s6[2]) - s6[5]), rc2);
+            k0 = HALF ? (near & 1u) != 0u : near != 0u;
+            k1 = HALF && (near & 2u) != 0u;
+            todo = false;
         }
         const unsigned tb = __ballot_sync(0xffffffffu, todo);
         const int rank = __popc(tb & below), n = __popc(tb);
@@ -774,19 +812,19 @@ __device__ __forceinline__ void prune_dev(const PruneArgs& A)
     }
 }
 
-template <int W, bool HALF>
+template <int W, bool HALF, bool WIDE>
 __global__ void __launch_bounds__(W == 1 ? 256 : 32 * W, W == 1 ? 4 : 32 / W) k_prune(PruneArgs A)
 {
-    prune_dev<W, HALF>(A);
+    prune_dev<W, HALF, WIDE>(A);
 }
 
-template <int W, bool HALF>
+template <int W, bool HALF, bool WIDE>
 __global__ void __launch_bounds__(W == 1 ? 256 : 32 * W, W == 1 ? 4 : 32 / W)
     k_prune_multi(const PruneArgs* __restrict__ As)
 {
     const PruneArgs& A = As[blockIdx.z];
     if ((int)blockIdx.x >= A.gx) return;
-    prune_dev<W, HALF>(A);
+    prune_dev<W, HALF, WIDE>(A);
 }
 
 // Warps per i cluster of a launch over ncl clusters: four where one each
@@ -868,19 +906,26 @@ static void launch_prune(void (*kern)(A), A arg, dim3 grid, int threads, bool se
     MDF_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, arg));
 }
 
-template <typename A>
-static void launch_prune_form(void (*w1)(A), void (*w1h)(A), void (*w4)(A), void (*w4h)(A), A arg, int warps, bool half,
-                              dim3 grid, bool selfp, cudaStream_t s)
+// The prune kernel of a form: single system (PruneArgs) or many (const PruneArgs*).
+template <bool WIDE>
+static auto prune_kernel(int warps, bool half) -> void (*)(PruneArgs)
 {
-    if (warps == 1) launch_prune(half ? w1h : w1, arg, grid, 256, selfp, s);
-    else launch_prune(half ? w4h : w4, arg, grid, 128, selfp, s);
+    if (warps == 1) return half ? k_prune<1, true, WIDE> : k_prune<1, false, WIDE>;
+    return half ? k_prune<4, true, WIDE> : k_prune<4, false, WIDE>;
+}
+template <bool WIDE>
+static auto prune_kernel_multi(int warps, bool half) -> void (*)(const PruneArgs*)
+{
+    if (warps == 1) return half ? k_prune_multi<1, true, WIDE> : k_prune_multi<1, false, WIDE>;
+    return half ? k_prune_multi<4, true, WIDE> : k_prune_multi<4, false, WIDE>;
 }
 
-// warps: the same in every system's arguments.
-void launch_prune_multi(const PruneArgs* d_args, int nsys, int gx, int warps, bool half, bool selfp, cudaStream_t s)
+// warps: the same in every system's arguments; wide: some FP64 system has wide clusters.
+void launch_prune_multi(const PruneArgs* d_args, int nsys, int gx, int warps, bool half, bool wide, bool selfp,
+                        cudaStream_t s)
 {
-    launch_prune_form<const PruneArgs*>(k_prune_multi<1, false>, k_prune_multi<1, true>, k_prune_multi<4, false>,
-                                        k_prune_multi<4, true>, d_args, warps, half, dim3(gx, 1, nsys), selfp, s);
+    launch_prune<const PruneArgs*>(wide ? prune_kernel_multi<true>(warps, half) : prune_kernel_multi<false>(warps, half),
+                                   d_args, dim3(gx, 1, nsys), warps == 1 ? 256 : 128, selfp, s);
 }
 
 // whole_entries: build the 8 x 8 pruned list even in the half layout (the
@@ -892,8 +937,8 @@ void prune_pairlist(Ctx& c, bool whole_entries)
     if (half) ensure_half_lists(c);
     const PruneArgs A = make_prune_args(c, half);
     if (A.ncl > 0)
-        launch_prune_form<PruneArgs>(k_prune<1, false>, k_prune<1, true>, k_prune<4, false>, k_prune<4, true>, A, A.warps,
-                                     half, grid_of(A), !A.force, c.stream);
+        launch_prune<PruneArgs>(prune_wide_clusters(c) ? prune_kernel<true>(A.warps, half) : prune_kernel<false>(A.warps, half),
+                                A, grid_of(A), A.warps == 1 ? 256 : 128, !A.force, c.stream);
     c.launches += 1;
     c.pruned_valid = true;
     c.pruned_half = half;
@@ -1089,10 +1134,10 @@ void build_pairlist(Ctx& c)
                 c.ilist.p, c.status.p);
             MDF_CUDA_TRY(cudaGetLastError());
             MDF_CUDA_TRY(cudaMemcpyAsync(c.h_build, d_ncl, sizeof(int), cudaMemcpyDeviceToHost, s));
-            MDF_CUDA_TRY(cudaMemcpyAsync(c.h_build + 1, c.d_build.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-            MDF_CUDA_TRY(cudaMemcpyAsync(c.h_build + 2, c.status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+            MDF_CUDA_TRY(cudaMemcpyAsync(c.h_build + 1, c.d_build.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+            MDF_CUDA_TRY(cudaMemcpyAsync(c.h_build + 3, c.status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
             MDF_CUDA_TRY(cudaStreamSynchronize(s));
-            st = (unsigned)c.h_build[2];
+            st = (unsigned)c.h_build[3];
             if (st & (ST_NONFINITE | ST_CAPACITY_COLUMN)) break;
             if (!(st & ST_CAPACITY_PAIRS)) break;
             // the list outgrew its buffer: grow to the count found (+1/8) and search again
@@ -1110,6 +1155,7 @@ void build_pairlist(Ctx& c)
         c.n_clusters = ncl;
         c.n_slots = ncl * CLUSTER;
         c.n_entries = c.h_build[1];
+        c.wide_clusters = c.h_build[2] != 0;
         c.cur_box.alloc(ncl);
         c.xq_f.alloc(c.n_slots);
         if (c.p.precision != MDF_PREC_MIXED) c.xq_d.alloc(c.n_slots);
