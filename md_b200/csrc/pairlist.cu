@@ -242,7 +242,8 @@ struct BoxF {
 };
 
 // Box of a cluster in absolute coordinates: centre, and half extents in units
-// of 2^(4s-6) A, rounded up, as 3 x 10 bits with s in the top two.
+// of 2^(6s-6) A, rounded up, as 3 x 10 bits with s in the top two (up to 4.1e6 A,
+// a box of 0.8 mm).
 __device__ __forceinline__ float4 box_encode(const float lo[3], const float hi[3], const double4& c, float pad)
 {
     float h[3], m = 0.f;
@@ -251,8 +252,8 @@ __device__ __forceinline__ float4 box_encode(const float lo[3], const float hi[3
         m = fmaxf(m, h[k]);
     }
     unsigned s = 0;
-    while (s < 3 && m > 1020.f * __uint_as_float((121u + 4u * s) << 23)) ++s;
-    const float per = __uint_as_float((133u - 4u * s) << 23);   // 2^(6-4s)
+    while (s < 3 && m > 1020.f * __uint_as_float((121u + 6u * s) << 23)) ++s;
+    const float per = __uint_as_float((133u - 6u * s) << 23);   // 2^(6-6s)
     unsigned u = s << 30;
     for (int k = 0; k < 3; ++k) u |= min(1023u, (unsigned)ceilf(h[k] * per)) << (10 * k);
     const bool real = lo[0] <= hi[0];
@@ -264,7 +265,7 @@ __device__ __forceinline__ float4 box_encode(const float lo[3], const float hi[3
 __device__ __forceinline__ BoxF box_decode(const float4& b)
 {
     const unsigned u = __float_as_uint(b.w);
-    const float unit = __uint_as_float((121u + 4u * (u >> 30)) << 23);
+    const float unit = __uint_as_float((121u + 6u * (u >> 30)) << 23);
     return BoxF{b.x, b.y, b.z, (float)(u & 1023u) * unit, (float)((u >> 10) & 1023u) * unit,
                 (float)((u >> 20) & 1023u) * unit, (u >> 30) == 0u};
 }

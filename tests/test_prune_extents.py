@@ -26,7 +26,7 @@ def _dimers(n, lx, spacing, seed=4):
 
 @pytest.mark.parametrize("layout", [0, 1])
 @pytest.mark.parametrize("n,lx,spacing", [(48, 26.0, 12.0), (48, 26.0, 40.0), (48, 26.0, 300.0), (48, 26.0, 1500.0),
-                                          (8500, 600.0, 15.0)])
+                                          (48, 26.0, 9000.0), (8500, 600.0, 15.0)])
 def test_fp64_prune_keeps_every_pair_of_long_clusters(n, lx, spacing, layout):
     x, q, box = _dimers(n, lx, spacing)
     w = x - box * np.floor(x / box)
