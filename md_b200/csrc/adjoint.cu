@@ -308,7 +308,6 @@ static void adj_consts(const Ctx& c, AdjArgs<float>& A)
     A.K = F.K;
     A.shifts = F.shifts;
     A.xq = c.xq_f.p;
-    A.vs = c.adj_vs_f.p;
 }
 static void adj_consts(const Ctx& c, AdjArgs<double>& A)
 {
@@ -317,14 +316,14 @@ static void adj_consts(const Ctx& c, AdjArgs<double>& A)
     A.shifts = F.shifts;
     A.poly = F.poly;
     A.xq = c.xq_d.p;
-    A.vs = c.adj_vs_d.p;
 }
 
 template <typename R>
-static void launch_adj_pairs(Ctx& c, const NBParams& P, double gE)
+static void launch_adj_pairs(Ctx& c, const NBParams& P, double gE, const AdjBufs& M)
 {
     AdjArgs<R> A{};
     adj_consts(c, A);
+    A.vs = reinterpret_cast<const typename V4<R>::type*>(M.vs);
     const bool pruned = c.p.prune_every != 0 && c.pruned_valid && !c.pruned_half;
     A.nlist = c.n_clusters;
     A.ilist = pruned ? c.ilist_in.p : c.ilist.p;
@@ -338,8 +337,8 @@ static void launch_adj_pairs(Ctx& c, const NBParams& P, double gE)
     A.hot[1] = c.hot_type[1];
     A.gE = (R)gE;
     A.kc = (R)P.kc;
-    A.dq_slot = c.adj_dq_slot.p;
-    A.dab = c.adj_dab.p;
+    A.dq_slot = M.dq_slot;
+    A.dab = M.dab;
     A.n_ljpair = c.n_ljpair;
     A.st = c.status.p;
     const size_t stage = (size_t)NB_WARPS * 4 * 2 * CLUSTER * (2 * sizeof(typename V4<R>::type) + sizeof(int));
@@ -363,6 +362,35 @@ static void launch_adj_pairs(Ctx& c, const NBParams& P, double gE)
     MDF_CUDA_TRY(cudaGetLastError());
 }
 
+// The call's buffers; slots by the list's capacity, so that a rebuilt list
+// rarely asks for more.
+static AdjBufs adj_bufs(Ctx& c)
+{
+    const bool mixed = c.p.precision == MDF_PREC_MIXED;
+    const size_t N = c.N, slots = c.slot_atom.n, ntot = (size_t)c.K[0] * c.K[1] * c.K[2];
+    const size_t nc = (size_t)c.K[0] * c.K[1] * (c.K[2] / 2 + 1);
+    const size_t bytes[8] = {sizeof(double) * 3 * N,
+                             (mixed ? sizeof(float4) : sizeof(double4)) * slots,
+                             sizeof(unsigned long long) * slots,
+                             sizeof(unsigned long long) * N,
+                             sizeof(double) * 2 * (size_t)c.n_ljpair,
+                             sizeof(double) * N,
+                             sizeof(unsigned long long) * ntot,
+                             (mixed ? sizeof(float2) : sizeof(double2)) * nc};
+    size_t off[9] = {0};
+    for (int i = 0; i < 8; ++i) off[i + 1] = off[i] + (bytes[i] + 255) / 256 * 256;
+    c.adj_mem.alloc(off[8]);
+    unsigned char* p = c.adj_mem.p;
+    return AdjBufs{reinterpret_cast<double*>(p + off[0]),
+                   p + off[1],
+                   reinterpret_cast<unsigned long long*>(p + off[2]),
+                   reinterpret_cast<unsigned long long*>(p + off[3]),
+                   reinterpret_cast<double*>(p + off[4]),
+                   reinterpret_cast<double*>(p + off[5]),
+                   reinterpret_cast<unsigned long long*>(p + off[6]),
+                   p + off[7]};
+}
+
 void backward(Ctx& c, const double* dL_dF, double dL_dE, double* dL_dq, double* dL_dA, double* dL_dB)
 {
     if (c.p.semantics != MDF_SEM_PHYSICAL)
@@ -377,8 +405,6 @@ void backward(Ctx& c, const double* dL_dF, double dL_dE, double* dL_dq, double* 
     if (dL_dF)
         for (long long i = 0; i < 3LL * c.N; ++i) scale = std::max(scale, std::fabs(dL_dF[i]));
     const int nlj = c.n_ljpair;
-    c.adj_dq.alloc(c.N);
-    c.adj_dab.alloc(2 * (size_t)std::max(nlj, 1));
     if (scale == 0.0 || !std::isfinite(scale)) {
         if (!std::isfinite(scale)) throw ApiError(MDF_ERR_NONFINITE, "non-finite dL/dF or dL/dE");
         if (dL_dq) std::fill(dL_dq, dL_dq + c.N, 0.0);
@@ -390,12 +416,11 @@ void backward(Ctx& c, const double* dL_dF, double dL_dE, double* dL_dq, double* 
     if (dL_dF)
         for (long long i = 0; i < 3LL * c.N; ++i) vn[i] = dL_dF[i] / scale;
     const double gE = dL_dE / scale;
-    c.adj_v.upload(vn.data(), vn.size(), s);
-    c.adj_dq_slot.alloc(c.n_slots);
-    c.adj_dq_atom.alloc(c.N);
-    MDF_CUDA_TRY(cudaMemsetAsync(c.adj_dq_slot.p, 0, sizeof(unsigned long long) * c.n_slots, s));
-    MDF_CUDA_TRY(cudaMemsetAsync(c.adj_dq_atom.p, 0, sizeof(unsigned long long) * c.N, s));
-    MDF_CUDA_TRY(cudaMemsetAsync(c.adj_dab.p, 0, sizeof(double) * 2 * std::max(nlj, 1), s));
+    const AdjBufs M = adj_bufs(c);
+    MDF_CUDA_TRY(cudaMemcpyAsync(M.v, vn.data(), sizeof(double) * vn.size(), cudaMemcpyHostToDevice, s));
+    MDF_CUDA_TRY(cudaMemsetAsync(M.dq_slot, 0, sizeof(unsigned long long) * c.n_slots, s));
+    MDF_CUDA_TRY(cudaMemsetAsync(M.dq_atom, 0, sizeof(unsigned long long) * c.N, s));
+    if (nlj > 0) MDF_CUDA_TRY(cudaMemsetAsync(M.dab, 0, sizeof(double) * 2 * nlj, s));
     MDF_CUDA_TRY(cudaMemsetAsync(c.status.p, 0, sizeof(unsigned), s));
     const int th = 256;
     // current cluster frame and pruned list, as a forward evaluation builds them
@@ -405,15 +430,12 @@ void backward(Ctx& c, const double* dL_dF, double dL_dE, double* dL_dq, double* 
         c.since_prune = 1;
         if (half_layout(c)) c.pruned_valid = false;   // the next forward prunes its half lists again
     }
-    if (mixed) {
-        c.adj_vs_f.alloc(c.n_slots);
-        k_adj_pack<float><<<grid_blocks(c.n_slots, th), th, 0, s>>>(c.n_slots, c.slot_atom.p, c.adj_v.p,
-                                                                     c.adj_vs_f.p);
-    } else {
-        c.adj_vs_d.alloc(c.n_slots);
-        k_adj_pack<double><<<grid_blocks(c.n_slots, th), th, 0, s>>>(c.n_slots, c.slot_atom.p, c.adj_v.p,
-                                                                      c.adj_vs_d.p);
-    }
+    if (mixed)
+        k_adj_pack<float><<<grid_blocks(c.n_slots, th), th, 0, s>>>(c.n_slots, c.slot_atom.p, M.v,
+                                                                     reinterpret_cast<float4*>(M.vs));
+    else
+        k_adj_pack<double><<<grid_blocks(c.n_slots, th), th, 0, s>>>(c.n_slots, c.slot_atom.p, M.v,
+                                                                      reinterpret_cast<double4*>(M.vs));
     const NBParams P = make_params(c);
     // the reciprocal-space part runs on the side stream, concurrently with
     // the pair adjoint (both only add into the fixed-point dq accumulators)
@@ -421,36 +443,36 @@ void backward(Ctx& c, const double* dL_dF, double dL_dE, double* dL_dq, double* 
     MDF_CUDA_TRY(cudaStreamWaitEvent(c.side, c.ev_fork, 0));
     c.stream = c.side;
     try {
-        pme_adjoint(c, gE, 1.0);
+        pme_adjoint(c, gE, M);
     } catch (...) {
         c.stream = s;
         throw;
     }
     c.stream = s;
     MDF_CUDA_TRY(cudaEventRecord(c.ev_join, c.side));
-    if (mixed) launch_adj_pairs<float>(c, P, gE);
-    else launch_adj_pairs<double>(c, P, gE);
+    if (mixed) launch_adj_pairs<float>(c, P, gE, M);
+    else launch_adj_pairs<double>(c, P, gE, M);
     if (c.n_excl + c.n_14 > 0)
         k_adj_pairs_fp64<<<grid_blocks(c.n_excl + c.n_14, th), th, 0, s>>>(
-            c.n_excl, c.excl_pairs.p, c.n_14, c.pairs14.p, c.p14_scale.p, c.xyz.p, c.q.p, c.adj_v.p, P, gE,
-            c.adj_dq_atom.p, c.status.p);
+            c.n_excl, c.excl_pairs.p, c.n_14, c.pairs14.p, c.p14_scale.p, c.xyz.p, c.q.p, M.v, P, gE,
+            M.dq_atom, c.status.p);
     MDF_CUDA_TRY(cudaStreamWaitEvent(s, c.ev_join, 0));
     // d/dq_a of gE (E_self + E_net): -2 k alpha/sqrt(pi) q_a and -k pi Q / (V alpha^2)
     const double V = c.box[0] * c.box[1] * c.box[2];
     const double self_coef = gE * (-2.0 * c.p.coulomb_const * c.alpha / std::sqrt(M_PI));
     const double net_coef = gE * (-c.p.coulomb_const * M_PI * c.q_total / (V * c.alpha * c.alpha));
-    k_adj_finish<<<grid_blocks(c.N, th), th, 0, s>>>(c.N, c.q.p, c.atom_slot.p, c.adj_dq_atom.p, c.adj_dq_slot.p,
-                                                     self_coef, net_coef, scale, c.adj_dq.p);
-    if (nlj > 0) k_scale<<<grid_blocks(2 * nlj, th), th, 0, s>>>(2 * nlj, c.adj_dab.p, scale);
+    k_adj_finish<<<grid_blocks(c.N, th), th, 0, s>>>(c.N, c.q.p, c.atom_slot.p, M.dq_atom, M.dq_slot, self_coef,
+                                                     net_coef, scale, M.dq);
+    if (nlj > 0) k_scale<<<grid_blocks(2 * nlj, th), th, 0, s>>>(2 * nlj, M.dab, scale);
     MDF_CUDA_TRY(cudaGetLastError());
     c.launches += 6;
     unsigned st = 0;
     MDF_CUDA_TRY(cudaMemcpyAsync(&st, c.status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    if (dL_dq) MDF_CUDA_TRY(cudaMemcpyAsync(dL_dq, c.adj_dq.p, sizeof(double) * c.N, cudaMemcpyDeviceToHost, s));
+    if (dL_dq) MDF_CUDA_TRY(cudaMemcpyAsync(dL_dq, M.dq, sizeof(double) * c.N, cudaMemcpyDeviceToHost, s));
     if (dL_dA && nlj > 0)
-        MDF_CUDA_TRY(cudaMemcpyAsync(dL_dA, c.adj_dab.p, sizeof(double) * nlj, cudaMemcpyDeviceToHost, s));
+        MDF_CUDA_TRY(cudaMemcpyAsync(dL_dA, M.dab, sizeof(double) * nlj, cudaMemcpyDeviceToHost, s));
     if (dL_dB && nlj > 0)
-        MDF_CUDA_TRY(cudaMemcpyAsync(dL_dB, c.adj_dab.p + nlj, sizeof(double) * nlj, cudaMemcpyDeviceToHost, s));
+        MDF_CUDA_TRY(cudaMemcpyAsync(dL_dB, M.dab + nlj, sizeof(double) * nlj, cudaMemcpyDeviceToHost, s));
     // the status word belongs to the forward's scalar block: leave it clear
     MDF_CUDA_TRY(cudaMemsetAsync(c.status.p, 0, sizeof(unsigned), s));
     MDF_CUDA_TRY(cudaStreamSynchronize(s));

@@ -843,8 +843,7 @@ void mdf_destroy(mdf_ctx* ctx)
             cudaStreamDestroy(cs);
         }
     c.d_build.release();
-    c.adj_v.release(); c.adj_vs_f.release(); c.adj_vs_d.release(); c.adj_dq_slot.release(); c.adj_dq_atom.release();
-    c.adj_dab.release(); c.adj_dq.release(); c.adj_qgrid.release(); c.adj_cgrid.release(); c.adj_rgrid.release();
+    c.adj_mem.release();
     if (c.md_exec) cudaGraphExecDestroy(c.md_exec);
     if (c.md_graph) cudaGraphDestroy(c.md_graph);
     if (c.md_host) cudaFreeHost(c.md_host);

@@ -340,7 +340,7 @@ __device__ __forceinline__ C* fft_to_last(int r1, int r2, const LineMap& M, cons
 }
 
 template <typename R>
-__device__ __forceinline__ void regs_z_r2c_dev(const FFTZArgs<R>& A, int bx)
+__device__ __forceinline__ void regs_z_r2c_dev(const FFTZArgs<R>& A, int bx, int set)
 {
     using C = typename CT<R>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -350,7 +350,8 @@ __device__ __forceinline__ void regs_z_r2c_dev(const FFTZArgs<R>& A, int bx)
     const C* tw = sm.tw;
     const LineMap M{LP, 1, n, false};
     const long long g0 = (long long)bx * 2 * LP;   // two real lines per complex one
-    const unsigned long long* __restrict__ q = A.qgrid;
+    const unsigned long long* __restrict__ q = set ? A.qgrid2 : A.qgrid;
+    C* __restrict__ cg = set ? A.cgrid2 : A.cgrid;
     auto value = [&](long long line, int z) {
         if (line >= nlines) return (R)0;
         const long long w = (long long)q[line * n + z];
@@ -370,13 +371,13 @@ __device__ __forceinline__ void regs_z_r2c_dev(const FFTZArgs<R>& A, int bx)
         const int l = (int)((unsigned)t / (unsigned)Kc), k = t - l * Kc;
         const C Z = out[l * n + k], Zc = cconj(out[l * n + (k == 0 ? 0 : n - k)]);
         const long long g = g0 + 2 * l;
-        if (g < nlines) A.cgrid[g * Kc + k] = C{(R)0.5 * (Z.x + Zc.x), (R)0.5 * (Z.y + Zc.y)};
-        if (g + 1 < nlines) A.cgrid[(g + 1) * Kc + k] = C{(R)0.5 * (Z.y - Zc.y), (R)-0.5 * (Z.x - Zc.x)};
+        if (g < nlines) cg[g * Kc + k] = C{(R)0.5 * (Z.x + Zc.x), (R)0.5 * (Z.y + Zc.y)};
+        if (g + 1 < nlines) cg[(g + 1) * Kc + k] = C{(R)0.5 * (Z.y - Zc.y), (R)-0.5 * (Z.x - Zc.x)};
     }
 }
 
 template <typename R>
-__device__ __forceinline__ void regs_z_c2r_dev(const FFTZArgs<R>& A, int bx)
+__device__ __forceinline__ void regs_z_c2r_dev(const FFTZArgs<R>& A, int bx, int set)
 {
     using C = typename CT<R>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -385,7 +386,8 @@ __device__ __forceinline__ void regs_z_c2r_dev(const FFTZArgs<R>& A, int bx)
     const C* tw = sm.tw;
     const LineMap M{LP, 1, n, false};
     const long long g0 = (long long)bx * 2 * LP;
-    const C* __restrict__ cg = A.cgrid;
+    const C* __restrict__ cg = set ? A.cgrid2 : A.cgrid;
+    R* __restrict__ rg = set ? A.rgrid2 : A.rgrid;
     const C* in = fft_to_last<true, R>(A.d.r[0], A.d.r[1], M, sm, [&](int l, int k) {
         const long long g = g0 + 2 * l;
         const int kk = k < Kc ? k : n - k;
@@ -409,14 +411,14 @@ __device__ __forceinline__ void regs_z_c2r_dev(const FFTZArgs<R>& A, int bx)
         const long long g = g0 + 2 * l;
 #pragma unroll
         for (int k = 0; k < (int)(sizeof(v) / sizeof(C)); ++k) {
-            if (g < nlines) A.rgrid[g * n + j + k * nb] = v[k].x;
-            if (g + 1 < nlines) A.rgrid[(g + 1) * n + j + k * nb] = v[k].y;
+            if (g < nlines) rg[g * n + j + k * nb] = v[k].x;
+            if (g + 1 < nlines) rg[(g + 1) * n + j + k * nb] = v[k].y;
         }
     });
 }
 
 template <typename R, bool INV>
-__device__ __forceinline__ void regs_y_dev(const FFTYArgs<R>& A, int bx, int by)
+__device__ __forceinline__ void regs_y_dev(const FFTYArgs<R>& A, int bx, int by, int set)
 {
     using C = typename CT<R>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -424,7 +426,7 @@ __device__ __forceinline__ void regs_y_dev(const FFTYArgs<R>& A, int bx, int by)
     const FftSmem<C> sm(smem_raw, n, LP, A.tw);
     const C* tw = sm.tw;
     const LineMap M{LP, LP, 1, true};
-    C* __restrict__ cg = A.cgrid + (long long)by * n * Kc + kz0;
+    C* __restrict__ cg = (set ? A.cgrid2 : A.cgrid) + (long long)by * n * Kc + kz0;
     const int live = min(LP, Kc - kz0);
     const C* in = fft_to_last<INV, R>(A.d.r[0], A.d.r[1], M, sm, [&](int l, int y) {
         return l < live ? cg[(long long)y * Kc + l] : C{0, 0};
@@ -438,18 +440,18 @@ __device__ __forceinline__ void regs_y_dev(const FFTYArgs<R>& A, int bx, int by)
 
 // The influence function is laid out [ky][kx][kz] here: lanes run along kz.
 template <typename R, bool ENERGY>
-__device__ __forceinline__ void regs_x_conv_dev(const FFTXArgs<R>& A, int bx, int by)
+__device__ __forceinline__ void regs_x_conv_dev(const FFTXArgs<R>& A, int bx, int by, int set)
 {
     using C = typename CT<R>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int n = A.d.n, Kc = A.Kc, K1 = A.K1, LP = A.LP, kz0 = bx * LP;
-    const int grid = by / K1, y = by - grid * K1;
+    const int y = by;
     const FftSmem<C> sm(smem_raw, n, LP, A.tw);
     C *const a = sm.a, *const b = sm.b;
     const C* tw = sm.tw;
     const LineMap M{LP, LP, 1, true};
     const long long stride = (long long)K1 * Kc;
-    C* __restrict__ cg = A.cgrid + grid * n * stride + (long long)y * Kc + kz0;
+    C* __restrict__ cg = (set ? A.cgrid2 : A.cgrid) + (long long)y * Kc + kz0;
     const R* __restrict__ fl = A.infl + (long long)y * n * Kc + kz0;
     const int live = min(LP, Kc - kz0);
     const int r1 = A.d.r[0], r2 = A.d.r[1], r3 = A.d.r[2];

@@ -315,13 +315,18 @@ struct GatherArgs {
     unsigned* st;
 };
 
-// z passes (r2c: charge grid -> half complex; c2r: half complex -> potential)
+// z passes (r2c: charge grid -> half complex; c2r: half complex -> potential).
+// A launch of gridDim.z = 2 transforms a second set of grids beside the first
+// (the adjoint's dipole chain); unused otherwise.
 template <typename R>
 struct FFTZArgs {
     int gx, gy;
     const unsigned long long* qgrid;              // r2c input
     typename V2<R>::type* cgrid;                   // r2c output / c2r input
     R* rgrid;                                      // c2r output
+    const unsigned long long* qgrid2;              // the second set
+    typename V2<R>::type* cgrid2;
+    R* rgrid2;
     int nlines;
     FFTDesc d;
     const typename V2<R>::type* tw;
@@ -332,7 +337,7 @@ struct FFTZArgs {
 template <typename R>
 struct FFTYArgs {
     int gx, gy;
-    typename V2<R>::type* cgrid;
+    typename V2<R>::type *cgrid, *cgrid2;
     int Kc;
     FFTDesc d;
     const typename V2<R>::type* tw;
@@ -344,7 +349,7 @@ struct FFTYArgs {
 template <typename R>
 struct FFTXArgs {
     int gx, gy;
-    typename V2<R>::type* cgrid;
+    typename V2<R>::type *cgrid, *cgrid2;
     int K1, Kc;
     FFTDesc d;
     const typename V2<R>::type* tw;

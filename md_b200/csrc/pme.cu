@@ -186,10 +186,10 @@ __device__ __forceinline__ void fft_smem_setup(unsigned char* raw, const FFTDesc
 
 // ------------------------------------------------------------- z passes
 template <typename R>
-__device__ __forceinline__ void fft_z_r2c_dev(const FFTZArgs<R>& A, int bx, int by)
+__device__ __forceinline__ void fft_z_r2c_dev(const FFTZArgs<R>& A, int bx, int by, int set)
 {
-    const unsigned long long* __restrict__ qgrid = A.qgrid;
-    typename CT<R>::type* __restrict__ cgrid = A.cgrid;
+    const unsigned long long* __restrict__ qgrid = set ? A.qgrid2 : A.qgrid;
+    typename CT<R>::type* __restrict__ cgrid = set ? A.cgrid2 : A.cgrid;
     const int nlines = A.nlines;
     const FFTDesc& dz = A.d;
     const typename CT<R>::type* __restrict__ twz = A.tw;
@@ -221,10 +221,10 @@ __device__ __forceinline__ void fft_z_r2c_dev(const FFTZArgs<R>& A, int bx, int 
 }
 
 template <typename R>
-__device__ __forceinline__ void fft_z_c2r_dev(const FFTZArgs<R>& A, int bx, int by)
+__device__ __forceinline__ void fft_z_c2r_dev(const FFTZArgs<R>& A, int bx, int by, int set)
 {
-    const typename CT<R>::type* __restrict__ cgrid = A.cgrid;
-    R* __restrict__ rgrid = A.rgrid;
+    const typename CT<R>::type* __restrict__ cgrid = set ? A.cgrid2 : A.cgrid;
+    R* __restrict__ rgrid = set ? A.rgrid2 : A.rgrid;
     const int nlines = A.nlines;
     const FFTDesc& dz = A.d;
     const typename CT<R>::type* __restrict__ twz = A.tw;
@@ -262,9 +262,9 @@ __device__ __forceinline__ void fft_z_c2r_dev(const FFTZArgs<R>& A, int bx, int 
 
 // ------------------------------------------------------------- y pass
 template <typename R>
-__device__ __forceinline__ void fft_y_dev(const FFTYArgs<R>& A, int bx, int by)
+__device__ __forceinline__ void fft_y_dev(const FFTYArgs<R>& A, int bx, int by, int set)
 {
-    typename CT<R>::type* __restrict__ cgrid = A.cgrid;
+    typename CT<R>::type* __restrict__ cgrid = set ? A.cgrid2 : A.cgrid;
     const int Kc = A.Kc;
     const FFTDesc& dy = A.d;
     const typename CT<R>::type* __restrict__ twy = A.tw;
@@ -298,9 +298,9 @@ __device__ __forceinline__ void fft_y_dev(const FFTYArgs<R>& A, int bx, int by)
 // ------------------------------------------- x pass + convolution + inverse
 
 template <typename R, bool ENERGY>
-__device__ __forceinline__ void fft_x_conv_dev(const FFTXArgs<R>& A, int bx, int by)
+__device__ __forceinline__ void fft_x_conv_dev(const FFTXArgs<R>& A, int bx, int by, int set)
 {
-    typename CT<R>::type* __restrict__ cgrid = A.cgrid;
+    typename CT<R>::type* __restrict__ cgrid = set ? A.cgrid2 : A.cgrid;
     const int K1 = A.K1, Kc = A.Kc;
     const FFTDesc& dx = A.d;
     const typename CT<R>::type* __restrict__ twx = A.tw;
@@ -319,10 +319,8 @@ __device__ __forceinline__ void fft_x_conv_dev(const FFTXArgs<R>& A, int bx, int
     int2* tab;
     fft_smem_setup(smem_raw, dx, twx, tabx, LP, tw, tab, bufA, bufB);
     const int K0 = dx.n;
-    // blocks past the first K1 rows take a second grid behind the first (the adjoint's two chains)
-    const int grid = by / K1, y = by - grid * K1, kz0 = bx * LP;
+    const int y = by, kz0 = bx * LP;
     const long long stride = (long long)K1 * Kc;
-    cgrid += grid * K0 * stride;
     for (int e = threadIdx.x; e < LP * K0; e += blockDim.x) {
         const int x = e >> lp_shift, l = e & (LP - 1), kz = kz0 + l;
         C v = {0, 0};
@@ -382,7 +380,7 @@ __device__ __forceinline__ void fft_x_conv_dev(const FFTXArgs<R>& A, int bx, int
     template <__VA_ARGS__>                                                                                    \
     __global__ void __launch_bounds__(FFT_THREADS) NAME(ARGS A)                                               \
     {                                                                                                         \
-        DEV(A, blockIdx.x, blockIdx.y);                                                                       \
+        DEV(A, blockIdx.x, blockIdx.y, blockIdx.z);                                                           \
     }                                                                                                         \
     template <__VA_ARGS__>                                                                                    \
     __global__ void __launch_bounds__(FFT_THREADS) NAME##_multi(const ARGS* __restrict__ As,                  \
@@ -390,7 +388,7 @@ __device__ __forceinline__ void fft_x_conv_dev(const FFTXArgs<R>& A, int bx, int
     {                                                                                                         \
         const int2 m = bmap[blockIdx.x];                                                                      \
         const ARGS& A = As[m.x];                                                                              \
-        DEV(A, m.y % A.gx, m.y / A.gx);                                                                       \
+        DEV(A, m.y % A.gx, m.y / A.gx, 0);                                                                    \
     }
 MDF_FFT_KERNELS(k_fft_z_r2c, fft_z_r2c_dev<R>, FFTZArgs<R>, typename R)
 MDF_FFT_KERNELS(k_fft_z_c2r, fft_z_c2r_dev<R>, FFTZArgs<R>, typename R)
@@ -400,7 +398,7 @@ MDF_FFT_KERNELS(k_fft_y, fft_y_dev<R>, FFTYArgs<R>, typename R)
 template <typename R, bool ENERGY>
 __global__ void __launch_bounds__(FFT_THREADS) k_fft_x_conv(FFTXArgs<R> A)
 {
-    fft_x_conv_dev<R, ENERGY>(A, blockIdx.x, blockIdx.y);
+    fft_x_conv_dev<R, ENERGY>(A, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // 64 registers (eight blocks per SM): the many-system grids are small and the
@@ -411,34 +409,37 @@ __global__ void __launch_bounds__(FFT_THREADS, 8) k_fft_x_conv_multi(const FFTXA
 {
     const int2 m = bmap[blockIdx.x];
     const FFTXArgs<R>& A = As[m.x];
-    fft_x_conv_dev<R, ENERGY>(A, m.y % A.gx, m.y / A.gx);
+    fft_x_conv_dev<R, ENERGY>(A, m.y % A.gx, m.y / A.gx, 0);
 }
 
 // The register-radix passes (fft_regs.cuh), same launch forms.
 template <typename R>
-__global__ void __launch_bounds__(FFT_THREADS) k_fftr_z_r2c(FFTZArgs<R> A) { regs_z_r2c_dev(A, blockIdx.x); }
+__global__ void __launch_bounds__(FFT_THREADS) k_fftr_z_r2c(FFTZArgs<R> A) { regs_z_r2c_dev(A, blockIdx.x, blockIdx.z); }
 template <typename R>
-__global__ void __launch_bounds__(FFT_THREADS) k_fftr_z_c2r(FFTZArgs<R> A) { regs_z_c2r_dev(A, blockIdx.x); }
+__global__ void __launch_bounds__(FFT_THREADS) k_fftr_z_c2r(FFTZArgs<R> A) { regs_z_c2r_dev(A, blockIdx.x, blockIdx.z); }
 template <typename R, bool INV>
-__global__ void __launch_bounds__(FFT_THREADS) k_fftr_y(FFTYArgs<R> A) { regs_y_dev<R, INV>(A, blockIdx.x, blockIdx.y); }
+__global__ void __launch_bounds__(FFT_THREADS) k_fftr_y(FFTYArgs<R> A)
+{
+    regs_y_dev<R, INV>(A, blockIdx.x, blockIdx.y, blockIdx.z);
+}
 template <typename R, bool ENERGY>
 __global__ void __launch_bounds__(FFT_THREADS) k_fftr_x_conv(FFTXArgs<R> A)
 {
-    regs_x_conv_dev<R, ENERGY>(A, blockIdx.x, blockIdx.y);
+    regs_x_conv_dev<R, ENERGY>(A, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 template <typename R>
 __global__ void __launch_bounds__(FFT_THREADS) k_fftr_z_r2c_multi(const FFTZArgs<R>* __restrict__ As,
                                                                   const int2* __restrict__ bmap)
 {
     const int2 m = bmap[blockIdx.x];
-    regs_z_r2c_dev(As[m.x], m.y);
+    regs_z_r2c_dev(As[m.x], m.y, 0);
 }
 template <typename R>
 __global__ void __launch_bounds__(FFT_THREADS) k_fftr_z_c2r_multi(const FFTZArgs<R>* __restrict__ As,
                                                                   const int2* __restrict__ bmap)
 {
     const int2 m = bmap[blockIdx.x];
-    regs_z_c2r_dev(As[m.x], m.y);
+    regs_z_c2r_dev(As[m.x], m.y, 0);
 }
 template <typename R, bool INV>
 __global__ void __launch_bounds__(FFT_THREADS) k_fftr_y_multi(const FFTYArgs<R>* __restrict__ As,
@@ -446,7 +447,7 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fftr_y_multi(const FFTYArgs<R>*
 {
     const int2 m = bmap[blockIdx.x];
     const FFTYArgs<R>& A = As[m.x];
-    regs_y_dev<R, INV>(A, m.y % A.gx, m.y / A.gx);
+    regs_y_dev<R, INV>(A, m.y % A.gx, m.y / A.gx, 0);
 }
 template <typename R, bool ENERGY>
 __global__ void __launch_bounds__(FFT_THREADS) k_fftr_x_conv_multi(const FFTXArgs<R>* __restrict__ As,
@@ -454,38 +455,50 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fftr_x_conv_multi(const FFTXArg
 {
     const int2 m = bmap[blockIdx.x];
     const FFTXArgs<R>& A = As[m.x];
-    regs_x_conv_dev<R, ENERGY>(A, m.y % A.gx, m.y / A.gx);
+    regs_x_conv_dev<R, ENERGY>(A, m.y % A.gx, m.y / A.gx, 0);
 }
 
-// One system's passes, each in the form its length has (d.r[0] != 0: register radices).
-template <typename R>
-static void launch_z_r2c(const FFTZArgs<R>& A, size_t sm, cudaStream_t s)
+// One system's passes, each in the form its length has (d.r[0] != 0: register
+// radices), over one set of grids or two.
+template <typename A>
+static dim3 grid_of_sets(const A& a, int sets)
 {
-    if (A.d.r[0]) k_fftr_z_r2c<R><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
-    else k_fft_z_r2c<R><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+    dim3 g = grid_of(a);
+    g.z = sets;
+    return g;
 }
 template <typename R>
-static void launch_z_c2r(const FFTZArgs<R>& A, size_t sm, cudaStream_t s)
+static void launch_z_r2c(const FFTZArgs<R>& A, size_t sm, cudaStream_t s, int sets = 1)
 {
-    if (A.d.r[0]) k_fftr_z_c2r<R><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
-    else k_fft_z_c2r<R><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+    const dim3 g = grid_of_sets(A, sets);
+    if (A.d.r[0]) k_fftr_z_r2c<R><<<g, FFT_THREADS, sm, s>>>(A);
+    else k_fft_z_r2c<R><<<g, FFT_THREADS, sm, s>>>(A);
 }
 template <typename R>
-static void launch_y(const FFTYArgs<R>& A, size_t sm, cudaStream_t s)
+static void launch_z_c2r(const FFTZArgs<R>& A, size_t sm, cudaStream_t s, int sets = 1)
 {
-    if (!A.d.r[0]) k_fft_y<R><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
-    else if (A.inverse) k_fftr_y<R, true><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
-    else k_fftr_y<R, false><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+    const dim3 g = grid_of_sets(A, sets);
+    if (A.d.r[0]) k_fftr_z_c2r<R><<<g, FFT_THREADS, sm, s>>>(A);
+    else k_fft_z_c2r<R><<<g, FFT_THREADS, sm, s>>>(A);
 }
 template <typename R>
-static void launch_x_conv(const FFTXArgs<R>& A, bool energy, size_t sm, cudaStream_t s)
+static void launch_y(const FFTYArgs<R>& A, size_t sm, cudaStream_t s, int sets = 1)
 {
+    const dim3 g = grid_of_sets(A, sets);
+    if (!A.d.r[0]) k_fft_y<R><<<g, FFT_THREADS, sm, s>>>(A);
+    else if (A.inverse) k_fftr_y<R, true><<<g, FFT_THREADS, sm, s>>>(A);
+    else k_fftr_y<R, false><<<g, FFT_THREADS, sm, s>>>(A);
+}
+template <typename R>
+static void launch_x_conv(const FFTXArgs<R>& A, bool energy, size_t sm, cudaStream_t s, int sets = 1)
+{
+    const dim3 g = grid_of_sets(A, sets);
     if (A.d.r[0]) {
-        if (energy) k_fftr_x_conv<R, true><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
-        else k_fftr_x_conv<R, false><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+        if (energy) k_fftr_x_conv<R, true><<<g, FFT_THREADS, sm, s>>>(A);
+        else k_fftr_x_conv<R, false><<<g, FFT_THREADS, sm, s>>>(A);
     } else {
-        if (energy) k_fft_x_conv<R, true><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
-        else k_fft_x_conv<R, false><<<grid_of(A), FFT_THREADS, sm, s>>>(A);
+        if (energy) k_fft_x_conv<R, true><<<g, FFT_THREADS, sm, s>>>(A);
+        else k_fft_x_conv<R, false><<<g, FFT_THREADS, sm, s>>>(A);
     }
 }
 
@@ -1116,6 +1129,9 @@ FFTChain<R> make_fft_chain(const Ctx& c, bool energy)
     F.zf.qgrid = c.qgrid.p;
     F.zf.cgrid = B.cg;
     F.zf.rgrid = B.rg;
+    F.zf.qgrid2 = nullptr;
+    F.zf.cgrid2 = nullptr;
+    F.zf.rgrid2 = nullptr;
     F.zf.nlines = nlines;
     F.zf.d = to_desc(c.plan[2]);
     F.zf.tw = B.twz;
@@ -1129,6 +1145,7 @@ FFTChain<R> make_fft_chain(const Ctx& c, bool energy)
     F.yf.gx = (Kc + LPy - 1) / LPy;
     F.yf.gy = K0;
     F.yf.cgrid = B.cg;
+    F.yf.cgrid2 = nullptr;
     F.yf.Kc = Kc;
     F.yf.d = to_desc(c.plan[1]);
     F.yf.tw = B.twy;
@@ -1145,6 +1162,7 @@ FFTChain<R> make_fft_chain(const Ctx& c, bool energy)
     F.x.gx = (Kc + LP - 1) / LP;
     F.x.gy = K1;
     F.x.cgrid = B.cg;
+    F.x.cgrid2 = nullptr;
     F.x.K1 = K1;
     F.x.Kc = Kc;
     F.x.d = to_desc(c.plan[0]);
@@ -1521,10 +1539,12 @@ template void launch_pme_multi<double>(const ZeroArgs*, BlockMap, const SpreadAr
 // C is symmetric, so C P is the same convolution chain applied to P.
 
 // The two chains run together: one spread fills the charge grid and the dipole
-// grid behind it, each FFT pass takes both in one launch, and one gather reads
-// both potentials - 8 launches instead of 16, on grids small enough that a
-// pass's time is mostly its latency.  At 28,000 atoms (72^3) the reciprocal
-// part's kernels went from 130 to 75 us in FP32, from 142 to 107 in FP64.
+// grid, each FFT pass takes both in one launch, and one gather reads both
+// potentials - 8 launches instead of 16, on grids small enough that a pass's
+// time is mostly its latency.  At 28,000 atoms (72^3) the reciprocal part's
+// kernels went from 130 to 75 us in FP32, from 142 to 107 in FP64.  The charge
+// chain runs through the context's own grids and leaves there what an
+// evaluation of these positions does; the dipole chain's are the adjoint's.
 
 // One derivative weight of the order-4 cardinal B-spline: dth[j] of bspline4.
 template <typename R>
@@ -1537,14 +1557,14 @@ __device__ __forceinline__ R dbspline4_one(R w, int j)
     return (R)0.5 * w2;
 }
 
-// Spread the charges onto qgrid and q_a (v_a . grad theta_a) onto the grid
-// ngrid words behind it, 16 lanes per atom as spread4_rows_dev.
+// Spread the charges onto qgrid and q_a (v_a . grad theta_a) onto dgrid, 16
+// lanes per atom as spread4_rows_dev.
 template <typename R>
 __global__ void __launch_bounds__(256) k_adj_spread(int nslots, const int* __restrict__ slot_atom,
                                                     const double* __restrict__ xyz, const double* __restrict__ q,
                                                     GridGeom g, const typename V4<R>::type* __restrict__ vs,
-                                                    unsigned long long* __restrict__ qgrid, long long ngrid,
-                                                    unsigned* st)
+                                                    unsigned long long* __restrict__ qgrid,
+                                                    unsigned long long* __restrict__ dgrid, unsigned* st)
 {
     const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int s = (int)(t0 >> 4);
@@ -1597,19 +1617,19 @@ __global__ void __launch_bounds__(256) k_adj_spread(int nslots, const int* __res
         int kx = base[0] - 1 + t;
         kx += (kx < 0) ? g.K[0] : 0;
         kx -= (kx >= g.K[0]) ? g.K[0] : 0;
-        unsigned long long* p = qgrid + ((long long)kx * g.K[1] + ky) * g.K[2] + kz;
+        const long long w = ((long long)kx * g.K[1] + ky) * g.K[2] + kz;
         const R val = qr * thx[t] * thy * thz;
         const R dip = (cx * dthx[t] * thy + cy * thx[t] * dthy) * thz + cz * thx[t] * thy * dthz;
-        atomicAdd(p, (unsigned long long)__double2ll_rn((double)val * GRID_SCALE));
-        atomicAdd(p + ngrid, (unsigned long long)__double2ll_rn((double)dip * GRID_SCALE));
+        atomicAdd(qgrid + w, (unsigned long long)__double2ll_rn((double)val * GRID_SCALE));
+        atomicAdd(dgrid + w, (unsigned long long)__double2ll_rn((double)dip * GRID_SCALE));
     }
 }
 
 // Per slot: gE phi - v . grad phi - (C P) at the atom, added to dq (fixed
-// point); C P lies ngrid values behind phi.
+// point).
 template <typename R>
 __global__ void k_adj_gather(int nslots, const int* __restrict__ slot_atom, const double* __restrict__ xyz,
-                             GridGeom g, const R* __restrict__ phi, long long ngrid,
+                             GridGeom g, const R* __restrict__ phi, const R* __restrict__ cpg,
                              const typename V4<R>::type* __restrict__ vs, double gE,
                              unsigned long long* __restrict__ dq, unsigned* st)
 {
@@ -1648,7 +1668,7 @@ __global__ void k_adj_gather(int nslots, const int* __restrict__ slot_atom, cons
                 const R v = phi[row + kz];
                 sz += th[2][k] * v;
                 dz += dth[2][k] * v;
-                cz += th[2][k] * phi[ngrid + row + kz];
+                cz += th[2][k] * cpg[row + kz];
             }
             const R tt = th[0][i] * th[1][j];
             p += tt * sz;
@@ -1666,48 +1686,41 @@ __global__ void k_adj_gather(int nslots, const int* __restrict__ slot_atom, cons
 }
 
 template <typename R>
-static void run_pme_adjoint(Ctx& c, double gE)
+static void run_pme_adjoint(Ctx& c, double gE, const AdjBufs& M)
 {
     using C = typename CT<R>::type;
     const PmeBufs<R> B(c);
-    const typename V4<R>::type* vs;
-    if (sizeof(R) == 4) vs = reinterpret_cast<const typename V4<R>::type*>(c.adj_vs_f.p);
-    else vs = reinterpret_cast<const typename V4<R>::type*>(c.adj_vs_d.p);
-    const int K0 = c.K[0], K1 = c.K[1], Kc = c.K[2] / 2 + 1;
-    const long long ntot = (long long)K0 * K1 * c.K[2];
-    c.adj_qgrid.alloc(2 * ntot);
-    c.adj_cgrid.alloc(sizeof(C) * 2 * (size_t)K0 * K1 * Kc);
-    c.adj_rgrid.alloc(sizeof(R) * 2 * (size_t)ntot);
-    R* rg = reinterpret_cast<R*>(c.adj_rgrid.p);
+    const typename V4<R>::type* vs = reinterpret_cast<const typename V4<R>::type*>(M.vs);
+    const long long ntot = (long long)c.K[0] * c.K[1] * c.K[2];
     const int th = 256;
-    MDF_CUDA_TRY(cudaMemsetAsync(c.adj_qgrid.p, 0, sizeof(unsigned long long) * 2 * ntot, c.stream));
+    MDF_CUDA_TRY(cudaMemsetAsync(c.qgrid.p, 0, sizeof(unsigned long long) * ntot, c.stream));
+    MDF_CUDA_TRY(cudaMemsetAsync(M.qgrid, 0, sizeof(unsigned long long) * ntot, c.stream));
     k_adj_spread<R><<<grid_blocks(16LL * c.n_slots, th), th, 0, c.stream>>>(
-        c.n_slots, c.slot_atom.p, c.xyz.p, c.q.p, B.g, vs, c.adj_qgrid.p, ntot, c.status.p);
+        c.n_slots, c.slot_atom.p, c.xyz.p, c.q.p, B.g, vs, c.qgrid.p, M.qgrid, c.status.p);
     FFTChain<R> F = make_fft_chain<R>(c, false);
-    F.zf.qgrid = c.adj_qgrid.p;
-    F.zf.cgrid = reinterpret_cast<C*>(c.adj_cgrid.p);
-    F.zf.rgrid = rg;
-    F.zf.nlines *= 2;
-    F.zf.gx = (F.zf.nlines + 2 * F.zf.LP - 1) / (2 * F.zf.LP);
-    F.zi = F.zf;
-    F.yf.cgrid = F.yi.cgrid = F.x.cgrid = F.zf.cgrid;
-    F.yf.gy = F.yi.gy = 2 * K0;
-    F.x.gy = 2 * K1;
-    launch_z_r2c(F.zf, F.smz, c.stream);
-    launch_y(F.yf, F.smy, c.stream);
-    launch_x_conv(F.x, false, F.smx, c.stream);
-    launch_y(F.yi, F.smy, c.stream);
-    launch_z_c2r(F.zi, F.smz, c.stream);
-    k_adj_gather<R><<<grid_blocks(c.n_slots, th), th, 0, c.stream>>>(c.n_slots, c.slot_atom.p, c.xyz.p, B.g, rg, ntot,
-                                                                      vs, gE, c.adj_dq_slot.p, c.status.p);
+    F.zf.qgrid2 = M.qgrid;
+    F.zf.cgrid2 = reinterpret_cast<C*>(M.cgrid);
+    // the dipole potential takes the place of the dipole grid, which nothing reads after the first pass
+    F.zf.rgrid2 = reinterpret_cast<R*>(M.qgrid);
+    F.zi.qgrid2 = F.zf.qgrid2;
+    F.zi.cgrid2 = F.zf.cgrid2;
+    F.zi.rgrid2 = F.zf.rgrid2;
+    F.yf.cgrid2 = F.yi.cgrid2 = F.x.cgrid2 = F.zf.cgrid2;
+    launch_z_r2c(F.zf, F.smz, c.stream, 2);
+    launch_y(F.yf, F.smy, c.stream, 2);
+    launch_x_conv(F.x, false, F.smx, c.stream, 2);
+    launch_y(F.yi, F.smy, c.stream, 2);
+    launch_z_c2r(F.zi, F.smz, c.stream, 2);
+    k_adj_gather<R><<<grid_blocks(c.n_slots, th), th, 0, c.stream>>>(
+        c.n_slots, c.slot_atom.p, c.xyz.p, B.g, B.rg, F.zf.rgrid2, vs, gE, M.dq_slot, c.status.p);
     MDF_CUDA_TRY(cudaGetLastError());
     c.launches += 7;
 }
 
-void pme_adjoint(Ctx& c, double gE, double)
+void pme_adjoint(Ctx& c, double gE, const AdjBufs& M)
 {
-    if (c.p.precision == MDF_PREC_MIXED) run_pme_adjoint<float>(c, gE);
-    else run_pme_adjoint<double>(c, gE);
+    if (c.p.precision == MDF_PREC_MIXED) run_pme_adjoint<float>(c, gE, M);
+    else run_pme_adjoint<double>(c, gE, M);
 }
 
 void launch_pme(Ctx& c, bool energy)
