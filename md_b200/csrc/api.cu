@@ -726,6 +726,13 @@ const char* mdf_last_error(const mdf_ctx* ctx)
 
 int mdf_create(const mdf_topology* top, const mdf_params* p, mdf_ctx** out)
 {
+    return mdf::create_context(top, p, nullptr, out);
+}
+
+}  // extern "C"
+
+int mdf::create_context(const mdf_topology* top, const mdf_params* p, const Ctx* like, mdf_ctx** out)
+{
     if (!out || !top || !p) {
         g_create_error = "null argument";
         return MDF_ERR_INVALID;
@@ -779,7 +786,10 @@ int mdf_create(const mdf_topology* top, const mdf_params* p, mdf_ctx** out)
         if (!(std::isfinite(c.alpha) && c.alpha >= 1e-12))
             throw ApiError(MDF_ERR_INVALID, "Ewald alpha must be finite and >= 1e-12 (ewald_tol in (0, 0.5))");
         if (c.p.precision == MDF_PREC_FP64 && c.p.semantics == MDF_SEM_PHYSICAL)
-            c.ewald_poly = make_ewald_poly(c.alpha, c.p.cutoff);
+            c.ewald_poly = like && like->p.precision == MDF_PREC_FP64 && like->alpha == c.alpha &&
+                                   like->p.cutoff == c.p.cutoff
+                               ? like->ewald_poly
+                               : make_ewald_poly(c.alpha, c.p.cutoff);
         upload_topology(c, top);
         if (!(c.box[0] > 0 && c.box[1] > 0 && c.box[2] > 0))
             throw ApiError(MDF_ERR_INVALID, "periodic box required");
@@ -798,6 +808,8 @@ int mdf_create(const mdf_topology* top, const mdf_params* p, mdf_ctx** out)
     *out = ctx;
     return MDF_OK;
 }
+
+extern "C" {
 
 void mdf_destroy(mdf_ctx* ctx)
 {

@@ -647,7 +647,7 @@ int mdf_batch_create(int nsys, const mdf_topology* const* topos, const mdf_param
             if (params[s].device != b->device) throw ApiError(MDF_ERR_INVALID, "all systems must use one device");
             if (params[s].semantics != MDF_SEM_PHYSICAL)
                 throw ApiError(MDF_ERR_UNSUPPORTED, "batches run PHYSICAL semantics");
-            int r = mdf_create(topos[s], &params[s], &b->sys[s]);
+            int r = create_context(topos[s], &params[s], s > 0 ? &b->sys[s - 1]->c : nullptr, &b->sys[s]);
             if (r != MDF_OK)
                 throw ApiError(r, "system " + std::to_string(s) + ": " + mdf_last_error(nullptr));
             const int len = 3 * b->sys[s]->c.N;

@@ -351,6 +351,8 @@ void minimize_lbfgs(Ctx& c, int max_iter, double fmax_tol, double max_step, int 
 void backward(Ctx& c, const double* dL_dF, double dL_dE, double* dL_dq, double* dL_dA, double* dL_dB);
 void pme_adjoint(Ctx& c, double gE, const AdjBufs& M);
 void build_pairlist(Ctx& c);
+// mdf_create; the Ewald polynomials of `like` (may be null) where alpha and cutoff agree
+int create_context(const mdf_topology* top, const mdf_params* p, const Ctx* like, mdf_ctx** out);
 void build_bands(Ctx& c);   // rank bands and halo plane lists of a split evaluation
 void pack_positions(Ctx& c);
 void prune_pairlist(Ctx& c, bool whole_entries = false);
