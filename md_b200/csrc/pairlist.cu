@@ -582,6 +582,7 @@ __global__ void __launch_bounds__(32 * SEARCH_WARPS) k_pair_search(
     }
     int held = 0;
     long long done = start;
+    __syncwarp();   // the first pass filled the buffer too
     generate([&](unsigned m, unsigned kk) {
         if (held + __popc(m) > SEARCH_CAP) {
             finish(held, done);
