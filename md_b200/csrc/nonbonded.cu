@@ -1132,7 +1132,7 @@ __global__ void __launch_bounds__(NB_THREADS, 2) k_pairs_f64(const __grid_consta
 }
 
 // Many systems with the same coefficients in one launch (a batch whose systems
-// differ in alpha or cutoff takes one launch per run of equal ones): passed by
+// differ in alpha or cutoff takes one launch per table, side by side): passed by
 // value they stay in the constant bank.  Read from each system's arguments or
 // from shared memory instead, 64 systems took 2.10 against 1.92 ms with exp
 // and erfc.
