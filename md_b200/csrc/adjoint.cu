@@ -324,7 +324,7 @@ static void launch_adj_pairs(Ctx& c, const NBParams& P, double gE, const AdjBufs
     AdjArgs<R> A{};
     adj_consts(c, A);
     A.vs = reinterpret_cast<const typename V4<R>::type*>(M.vs);
-    const bool pruned = c.p.prune_every != 0 && c.pruned_valid && !c.pruned_half;
+    const bool pruned = c.p.prune_every != 0;   // backward() has just pruned whole entries
     A.nlist = c.n_clusters;
     A.ilist = pruned ? c.ilist_in.p : c.ilist.p;
     A.plist = pruned ? c.plist_in.p : c.plist.p;
