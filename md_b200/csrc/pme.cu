@@ -77,7 +77,9 @@ __device__ __forceinline__ void small_dft(C* v, int Rr, bool inverse, const C* t
         v[2].x = m2.x - n2.y; v[2].y = m2.y + n2.x;
         v[3].x = m2.x + n2.y; v[3].y = m2.y - n2.x;
     } else {
-        // generic prime radix through the line's twiddle table: W_R^q = W_n^{q n/R}
+        // generic prime radix through the line's twiddle table: W_R^q = W_n^{q n/R};
+        // fused by hand (cmul_fixed), so that every kernel it is inlined in - one
+        // system's and a batch's - rounds alike
         C out[32];
         const int step = n / Rr;
         for (int t = 0; t < Rr; ++t) {
@@ -85,9 +87,8 @@ __device__ __forceinline__ void small_dft(C* v, int Rr, bool inverse, const C* t
             for (int r = 0; r < Rr; ++r) {
                 C w = tw[((r * t) % Rr) * step];
                 if (inverse) w = cconj(w);
-                C p = cmul(v[r], w);
-                acc.x += p.x;
-                acc.y += p.y;
+                acc.x = fma(-v[r].y, w.y, fma(v[r].x, w.x, acc.x));
+                acc.y = fma(v[r].y, w.x, fma(v[r].x, w.y, acc.y));
             }
             out[t] = acc;
         }
@@ -121,6 +122,15 @@ __device__ __forceinline__ void stage_fixed(const C* in, C* out, int n, int Ns, 
     }
 }
 
+// Complex product with its roundings spelled out: the compiler chooses which
+// product of cmul it fuses, and chose differently for one system and for many.
+template <typename C, typename R>
+__device__ __forceinline__ C cmul_fixed(C a, C b)
+{
+    const R x = mul_rn(a.y, b.y), y = mul_rn(a.y, b.x);
+    return C{fma(a.x, b.x, -x), fma(a.x, b.y, y)};
+}
+
 template <typename C, typename R>
 __device__ void stage_generic(const C* in, C* out, int n, int Rr, int Ns, const C* tw, const int2* tab, int lt,
                               int tpl, bool inverse)
@@ -134,7 +144,7 @@ __device__ void stage_generic(const C* in, C* out, int n, int Rr, int Ns, const 
             if (r && t.x) {
                 C w = tw[r * t.x];
                 if (inverse) w = cconj(w);
-                x = cmul(x, w);
+                x = cmul_fixed<C, R>(x, w);
             }
             v[r] = x;
         }
