@@ -359,17 +359,17 @@ void upload_topology(Ctx& c, const mdf_topology* t)
     c.excl_pairs.upload(ex.data(), ex.size(), s);
     c.excl_is14.upload(is14.data(), is14.size(), s);
     if (c.n_excl > 0) {
-        std::vector<int> off(c.N + 1, 0), nb(ex.size());
-        for (int a : ex) ++off[a + 1];
-        for (int i = 0; i < c.N; ++i) off[i + 1] += off[i];
-        std::vector<int> at(off.begin(), off.end() - 1);
+        // the partners' rows behind their N + 1 offsets, in one upload
+        std::vector<int> rows(c.N + 1 + ex.size(), 0);
+        int* nb = rows.data() + c.N + 1;
+        for (int a : ex) ++rows[a + 1];
+        for (int i = 0; i < c.N; ++i) rows[i + 1] += rows[i];
+        std::vector<int> at(rows.begin(), rows.begin() + c.N);
         for (size_t i = 0; i < ex.size(); i += 2) {
             nb[at[ex[i]]++] = ex[i + 1];
             nb[at[ex[i + 1]]++] = ex[i];
         }
-        c.ex_off.upload(off.data(), off.size(), s);
-        c.ex_nb.upload(nb.data(), nb.size(), s);
-        MDF_CUDA_TRY(cudaStreamSynchronize(s));
+        c.ex_rows.upload(rows.data(), rows.size(), s);
     }
     {
         std::vector<int> p(2 * (size_t)c.n_14);
@@ -826,7 +826,7 @@ void mdf_destroy(mdf_ctx* ctx)
     c.bond_atoms.release(); c.ub_atoms.release(); c.angle_atoms.release(); c.dih_atoms.release();
     c.imp_atoms.release(); c.cmap_atoms.release(); c.cmap_set.release(); c.bond_par.release(); c.ub_par.release();
     c.angle_par.release(); c.imp_par.release(); c.dih_par.release(); c.cmap_coeff.release();
-    c.excl_pairs.release(); c.pairs14.release(); c.p14_scale.release(); c.excl_is14.release(); c.ex_off.release(); c.ex_nb.release();
+    c.excl_pairs.release(); c.pairs14.release(); c.p14_scale.release(); c.excl_is14.release(); c.ex_rows.release();
     c.xyz.release(); c.atom_col.release(); c.col_count.release(); c.col_start.release(); c.col_cstart.release();
     c.col_atoms.release(); c.slot_atom.release(); c.atom_slot.release(); c.slot_type.release(); c.center.release(); c.centerf.release();
     c.bb_lo.release(); c.bb_hi.release(); c.xq_f.release(); c.xq_d.release(); c.cluster_col.release();

@@ -149,7 +149,7 @@ struct Ctx {
     DevBuf<double4> ljAB4_d;       // the same in FP64 (FP64 PHYSICAL pair kernel)
     DevBuf<double2> lj14AB;    // same indexing, 1-4 tables
     DevBuf<int> ljvalid;       // [(ntypes+1)^2] nb != 0
-    DevBuf<int> ex_off, ex_nb; // each atom's excluded partners: ex_nb[ex_off[a] .. ex_off[a + 1])
+    DevBuf<int> ex_rows;       // each atom's excluded partners: N + 1 offsets, then the rows
     int hot_type[2] = {0, 0};  // the two most frequent atom types
     EwaldPoly ewald_poly{};    // FP64 PHYSICAL contexts
     int ntp = 0;               // ntypes + 1 (padding type appended)

@@ -1132,8 +1132,8 @@ void build_pairlist(Ctx& c)
             MDF_CUDA_TRY(cudaMemsetAsync(c.d_build.p, 0, sizeof(int) * 4, s));
             k_pair_search<<<grid_blocks(ncl_cap, SEARCH_WARPS), 32 * SEARCH_WARPS, 0, s>>>(
                 d_ncl, g, c.cluster_col.p, c.col_cstart.p, c.bb_lo.p, c.bb_hi.p, c.center.p, c.slot_atom.p,
-                c.atom_slot.p, c.xyz.p, c.n_excl > 0 ? c.ex_off.p : nullptr, c.ex_nb.p, c.d_build.p, c.plist.p, cap,
-                c.ilist.p, c.status.p);
+                c.atom_slot.p, c.xyz.p, c.n_excl > 0 ? c.ex_rows.p : nullptr,
+                c.n_excl > 0 ? c.ex_rows.p + c.N + 1 : nullptr, c.d_build.p, c.plist.p, cap, c.ilist.p, c.status.p);
             MDF_CUDA_TRY(cudaGetLastError());
             MDF_CUDA_TRY(cudaMemcpyAsync(c.h_build, d_ncl, sizeof(int), cudaMemcpyDeviceToHost, s));
             MDF_CUDA_TRY(cudaMemcpyAsync(c.h_build + 1, c.d_build.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
