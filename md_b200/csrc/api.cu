@@ -404,6 +404,17 @@ void allreduce_u64(Ctx& c, unsigned long long* d, long long n)
         throw ApiError(MDF_ERR_CUDA, "the allreduce callback failed");
 }
 
+// The stream of the listed terms: made with the context, except in a batch,
+// whose many-system launches have streams of their own (0.08 ms a context).
+void ensure_side2(Ctx& c)
+{
+    if (c.side2) return;
+    int lo = 0, hi = 0;
+    MDF_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    MDF_CUDA_TRY(cudaStreamCreateWithPriority(&c.side2, cudaStreamNonBlocking, hi));
+    MDF_CUDA_TRY(cudaEventCreateWithFlags(&c.ev_join2, cudaEventDisableTiming));
+}
+
 void eval_async_impl(Ctx& c, uint32_t flags)
 {
     if (!c.have_positions) throw ApiError(MDF_ERR_STATE, "positions not set");
@@ -427,8 +438,11 @@ void eval_async_impl(Ctx& c, uint32_t flags)
     // kernel; the main stream waits for them before k_finalize.  With timing enabled every
     // kernel runs on the main stream so the per-phase times are separable.
     const bool want_pme = phys || (flags & MDF_COMPUTE_PME_REFERENCE);
-    const bool overlap = want_pme && !c.timing;
-    if (overlap) MDF_CUDA_TRY(cudaEventRecord(c.ev_fork, s));
+    const bool overlap = want_pme && !c.timing && !c.one_stream;
+    if (overlap) {
+        ensure_side2(c);
+        MDF_CUDA_TRY(cudaEventRecord(c.ev_fork, s));
+    }
     // the main stream's kernels go first: the pair kernel ends the evaluation of
     // all but small systems, and the host's launches of the side streams would
     // hold its chain back (the side stream's priority places its blocks anyway)
@@ -726,12 +740,12 @@ const char* mdf_last_error(const mdf_ctx* ctx)
 
 int mdf_create(const mdf_topology* top, const mdf_params* p, mdf_ctx** out)
 {
-    return mdf::create_context(top, p, nullptr, out);
+    return mdf::create_context(top, p, false, nullptr, out);
 }
 
 }  // extern "C"
 
-int mdf::create_context(const mdf_topology* top, const mdf_params* p, const Ctx* like, mdf_ctx** out)
+int mdf::create_context(const mdf_topology* top, const mdf_params* p, bool in_batch, const Ctx* like, mdf_ctx** out)
 {
     if (!out || !top || !p) {
         g_create_error = "null argument";
@@ -770,11 +784,10 @@ int mdf::create_context(const mdf_topology* top, const mdf_params* p, const Ctx*
             int lo = 0, hi = 0;
             MDF_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));
             MDF_CUDA_TRY(cudaStreamCreateWithPriority(&c.side, cudaStreamNonBlocking, hi));
-            MDF_CUDA_TRY(cudaStreamCreateWithPriority(&c.side2, cudaStreamNonBlocking, hi));
         }
         MDF_CUDA_TRY(cudaEventCreateWithFlags(&c.ev_fork, cudaEventDisableTiming));
         MDF_CUDA_TRY(cudaEventCreateWithFlags(&c.ev_join, cudaEventDisableTiming));
-        MDF_CUDA_TRY(cudaEventCreateWithFlags(&c.ev_join2, cudaEventDisableTiming));
+        if (!in_batch) ensure_side2(c);
         MDF_CUDA_TRY(cudaHostAlloc((void**)&c.h_scal, sizeof(unsigned long long) * NUM_SCAL, cudaHostAllocMapped));
         memset(c.h_scal, 0, sizeof(unsigned long long) * NUM_SCAL);
         MDF_CUDA_TRY(cudaHostGetDevicePointer((void**)&c.d_hscal, c.h_scal, 0));

@@ -517,6 +517,7 @@ void build_lists(mdf_batch* b)
 {
     if (!b->have_positions) throw ApiError(MDF_ERR_STATE, "positions not set");
     drop_graph(b);
+    const bool multi = uniform_launches(b);   // the contexts' own chains are not used again
     for (int s = 0; s < b->nsys; ++s) {
         Ctx& c = b->sys[s]->c;
         MDF_CUDA_TRY(cudaMemcpyAsync(c.xyz.p, b->h_pos + b->off[s], sizeof(double) * 3 * (size_t)c.N,
@@ -525,6 +526,7 @@ void build_lists(mdf_batch* b)
         build_pairlist(c);
         // one plain evaluation: clears the accumulators and counts pairs, so
         // the captured evaluations need no first-use work
+        c.one_stream = multi;
         eval_async_impl(c, MDF_COMPUTE_ENERGY | MDF_COMPUTE_FORCES);
     }
     for (int s = 0; s < b->nsys; ++s) MDF_CUDA_TRY(cudaStreamSynchronize(b->sys[s]->c.stream));
@@ -666,7 +668,7 @@ int mdf_batch_create(int nsys, const mdf_topology* const* topos, const mdf_param
             if (params[s].device != b->device) throw ApiError(MDF_ERR_INVALID, "all systems must use one device");
             if (params[s].semantics != MDF_SEM_PHYSICAL)
                 throw ApiError(MDF_ERR_UNSUPPORTED, "batches run PHYSICAL semantics");
-            int r = create_context(topos[s], &params[s], s > 0 ? &b->sys[s - 1]->c : nullptr, &b->sys[s]);
+            int r = create_context(topos[s], &params[s], true, s > 0 ? &b->sys[s - 1]->c : nullptr, &b->sys[s]);
             if (r != MDF_OK)
                 throw ApiError(r, "system " + std::to_string(s) + ": " + mdf_last_error(nullptr));
             const int len = 3 * b->sys[s]->c.N;

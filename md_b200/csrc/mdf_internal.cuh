@@ -133,7 +133,8 @@ struct Ctx {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaStream_t side = nullptr;         // the PME chain runs here, concurrently with the pair kernel
-    cudaStream_t side2 = nullptr;        // the listed FP64 terms run here
+    cudaStream_t side2 = nullptr;        // the listed FP64 terms run here (ensure_side2)
+    bool one_stream = false;             // evaluate on `stream` alone
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr;
     mdf_params p{};
     int N = 0;
@@ -351,8 +352,9 @@ void minimize_lbfgs(Ctx& c, int max_iter, double fmax_tol, double max_step, int 
 void backward(Ctx& c, const double* dL_dF, double dL_dE, double* dL_dq, double* dL_dA, double* dL_dB);
 void pme_adjoint(Ctx& c, double gE, const AdjBufs& M);
 void build_pairlist(Ctx& c);
-// mdf_create; the Ewald polynomials of `like` (may be null) where alpha and cutoff agree
-int create_context(const mdf_topology* top, const mdf_params* p, const Ctx* like, mdf_ctx** out);
+// mdf_create; in_batch: without the stream of the listed terms; the Ewald
+// polynomials of `like` (may be null) where alpha and cutoff agree
+int create_context(const mdf_topology* top, const mdf_params* p, bool in_batch, const Ctx* like, mdf_ctx** out);
 void build_bands(Ctx& c);   // rank bands and halo plane lists of a split evaluation
 void pack_positions(Ctx& c);
 void prune_pairlist(Ctx& c, bool whole_entries = false);
