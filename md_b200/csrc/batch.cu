@@ -281,7 +281,7 @@ MultiDev<R> prepare_multi(mdf_batch* b, uint32_t flags, MultiArgs<R>& M, double*
         }
         M.pack.push_back(make_pack_args<R>(c));
         M.prune.push_back(make_prune_args(c, M.half));
-        M.prune_wide = M.prune_wide || prune_wide_clusters(c);
+        M.prune_wide = M.prune_wide || c.wide_clusters;
         if (sizeof(R) == 4) {
             size_t dyn = 0;
             M.pf32.push_back(make_pair_f32_args(c, &dyn));

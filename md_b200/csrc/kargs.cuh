@@ -53,7 +53,7 @@ struct PruneArgs {
     const ILRange* ilist;
     const PairEntry* plist;
     const float4* xf;
-    const double4* xd;      // FP64 contexts: the offsets in FP64 (snap_d, wide clusters)
+    const double4* xd;      // FP64 contexts: the offsets in FP64 (snap_d, wide clusters); mixed: null
     const float4 *centerf, *box;
     int box_fine;           // box padding small enough for the acceptance by boxes
     ShiftTable shifts;

@@ -358,8 +358,6 @@ int create_context(const mdf_topology* top, const mdf_params* p, bool in_batch, 
 void build_bands(Ctx& c);   // rank bands and halo plane lists of a split evaluation
 void pack_positions(Ctx& c);
 void prune_pairlist(Ctx& c, bool whole_entries = false);
-// the prune tests wide clusters in FP64
-inline bool prune_wide_clusters(const Ctx& c) { return c.wide_clusters && c.p.precision != MDF_PREC_MIXED; }
 // half-entry lists in use by the pair kernel (layout 1, pruned)
 inline bool half_layout(const Ctx& c) { return c.p.pair_layout == 1 && c.p.prune_every != 0; }
 // prune_every < 0: the device prunes when an atom moved more than prune_margin / 2

@@ -401,9 +401,9 @@ __device__ __forceinline__ bool excluded_entry(int I, int la, int a, int b, cons
     return true;
 }
 
-// Clusters beyond this extent (A) are pruned by the WIDE form in FP64 contexts;
-// below it, whatever the atoms move until the next build, the FP32 test's
-// rounding stays near 1e-2 A^2.  Liquids stay at 5 to 10 A.
+// Clusters beyond this extent (A) are pruned by the WIDE form; below it, whatever
+// the atoms move until the next build, the FP32 test's rounding stays near 1e-2
+// A^2.  Liquids stay at 5 to 10 A.
 constexpr float WIDE_EXTENT = 64.f;
 
 constexpr int SEARCH_WARPS = 4;
@@ -605,9 +605,9 @@ __global__ void __launch_bounds__(32 * SEARCH_WARPS) k_pair_search(
 // rounds with the square of the clusters' extents, by ~1e-4 A^2 at liquid
 // density and ~2e-3 A^2 at half extents of 16 A (BoxF.fine), inside the radius'
 // 0.02 A margin (0.1 A^2 at a cutoff of 3 A).  Wider clusters, those of very
-// dilute systems, lose pairs near the cutoff from extents of some hundred A on:
-// FP64 contexts that have them test their entries in FP64 (WIDE, prune_wide),
-// mixed contexts don't.
+// dilute systems, would lose pairs near the cutoff from extents of some hundred
+// A on: where there are some, their entries are tested without the expansion, in
+// the precision of the positions (WIDE, prune_wide).
 //
 // W warps share an i cluster (32 entries each per round).  An entry is first
 // tested lane by lane through the clusters' current boxes (k_pack): farther
@@ -648,19 +648,21 @@ __device__ __forceinline__ float min_with2(float m, F32x2 v)   // min(m, v.lo, v
 
 constexpr int PRUNE_WARPS = 8;   // largest block
 
-// One entry in FP64, without the expansion: bit h set when half h of the i
-// cluster has an atom pair within the radius.  Called for clusters too wide for
-// the FP32 test; not inlined, so that it takes no registers from it.
-__device__ __noinline__ unsigned prune_wide(const double4* __restrict__ xi, const double4* __restrict__ xj, float ox,
-                                            float oy, float oz, float rc2)
+// One entry without the expansion: bit h set when half h of the i cluster has an
+// atom pair within the radius.  Called for clusters too wide for the FP32 test;
+// not inlined, so that it takes no registers from it.
+template <typename R>
+__device__ __noinline__ unsigned prune_wide(const typename V4<R>::type* __restrict__ xi,
+                                            const typename V4<R>::type* __restrict__ xj, float ox, float oy, float oz,
+                                            float rc2)
 {
     unsigned near = 0;
     for (int j = 0; j < CLUSTER && near != 3u; ++j) {
-        const double4 b = xj[j];
-        const double qx = b.x + ox, qy = b.y + oy, qz = b.z + oz;
+        const typename V4<R>::type b = xj[j];
+        const R qx = b.x + ox, qy = b.y + oy, qz = b.z + oz;
         for (int i = 0; i < CLUSTER; ++i) {
-            const double4 a = xi[i];
-            const double dx = a.x - qx, dy = a.y - qy, dz = a.z - qz;
+            const typename V4<R>::type a = xi[i];
+            const R dx = a.x - qx, dy = a.y - qy, dz = a.z - qz;
             if (fma(dx, dx, fma(dy, dy, dz * dz)) < rc2) near |= 1u << (i / 4);
         }
     }
@@ -734,9 +736,11 @@ __device__ __forceinline__ void prune_dev(const PruneArgs& A)
         }
         if (WIDE && todo && !(bi.fine && bj.fine)) {
             const float4 cJ = A.centerf[my.j];
-            const unsigned near = prune_wide(A.xd + (size_t)I * CLUSTER, A.xd + (size_t)my.j * CLUSTER,
-                                             -(((cI.x - cJ.x) - s6[0]) - s6[3]), -(((cI.y - cJ.y) - s6[1]) - s6[4]),
-                                             -(((cI.z - cJ.z) - s6[2]) - s6[5]), rc2);
+            const float ox = -(((cI.x - cJ.x) - s6[0]) - s6[3]), oy = -(((cI.y - cJ.y) - s6[1]) - s6[4]),
+                        oz = -(((cI.z - cJ.z) - s6[2]) - s6[5]);
+            const size_t si = (size_t)I * CLUSTER, sj = (size_t)my.j * CLUSTER;
+            const unsigned near = A.xd ? prune_wide<double>(A.xd + si, A.xd + sj, ox, oy, oz, rc2)
+                                       : prune_wide<float>(xf + si, xf + sj, ox, oy, oz, rc2);
             k0 = HALF ? (near & 1u) != 0u : near != 0u;
             k1 = HALF && (near & 2u) != 0u;
             todo = false;
@@ -922,7 +926,7 @@ static auto prune_kernel_multi(int warps, bool half) -> void (*)(const PruneArgs
     return half ? k_prune_multi<4, true, WIDE> : k_prune_multi<4, false, WIDE>;
 }
 
-// warps: the same in every system's arguments; wide: some FP64 system has wide clusters.
+// warps: the same in every system's arguments; wide: some system has wide clusters.
 void launch_prune_multi(const PruneArgs* d_args, int nsys, int gx, int warps, bool half, bool wide, bool selfp,
                         cudaStream_t s)
 {
@@ -939,7 +943,7 @@ void prune_pairlist(Ctx& c, bool whole_entries)
     if (half) ensure_half_lists(c);
     const PruneArgs A = make_prune_args(c, half);
     if (A.ncl > 0)
-        launch_prune<PruneArgs>(prune_wide_clusters(c) ? prune_kernel<true>(A.warps, half) : prune_kernel<false>(A.warps, half),
+        launch_prune<PruneArgs>(c.wide_clusters ? prune_kernel<true>(A.warps, half) : prune_kernel<false>(A.warps, half),
                                 A, grid_of(A), A.warps == 1 ? 256 : 128, !A.force, c.stream);
     c.launches += 1;
     c.pruned_valid = true;
