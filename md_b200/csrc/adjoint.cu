@@ -110,9 +110,8 @@ __device__ __forceinline__ double adj_rc(const PairConstD& K) { return K.rc; }
 // fixed, so its pairs with the two most frequent atom types (of a solvated
 // system, nearly all pairs) have two entries known before the loop: their sums
 // stay in registers, and only pairs with other types add to the block's sums
-// in shared memory at once.  Summing runs of one entry and flushing at each
-// change, as before, met a change at almost every pair, 32 lanes adding to a
-// handful of shared words.
+// in shared memory at once.  (Runs of one entry, flushed when it changes, change
+// at almost every pair, 32 lanes adding to a handful of shared words.)
 //
 // What bounds it: issue in FP32, the double-precision pipe in FP64.  28,000
 // atoms: FP32 250 -> 93 us, FP64 521 -> 205 us (with the Ewald polynomials).

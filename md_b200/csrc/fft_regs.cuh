@@ -510,7 +510,7 @@ __device__ __forceinline__ void regs_x_conv_dev(const FFTXArgs<R>& A, int bx, in
                     if (energy && c[u] != (R)0) {
                         const double em = (double)c[u] * ((double)S.x * S.x + (double)S.y * S.y);
                         const double m2 = fma(mx[u], mx[u], myz2);
-                        double r = (double)rcp_ftz((float)m2);   // and two Newton steps: 1/m2
+                        double r = (double)rcp_ftz((float)m2);   // 1/m2: Newton's iteration r (2 - m2 r), twice
                         r = fma(r, fma(-m2, r, 1.0), r);
                         r = fma(r, fma(-m2, r, 1.0), r);
                         const double h = em * r;

@@ -155,11 +155,12 @@ struct PairF64Args {
 // instruction takes it two cycles), and exp and erfc were more than half of
 // what a pair put on it.  Over the cutoff's range both terms are 1/r and 1/r^3
 // minus one polynomial each in r^2 (ewald_poly.hpp; 2-5e-16 of the largest
-// value): 26 FMAs instead of exp + erfc, half of them when only forces are
-// wanted, and coefficients that the FMA reads from the constant bank.  Slots
-// outside the cutoff give finite values that the caller drops.  With an
-// alpha rc beyond EWALD_Z_MAX (ewald_tol below 1e-6) the functions themselves
-// are called.  Pair launch at 100k atoms (half lists, energies)
+// value): 52 FMAs instead of exp + erfc, 26 when only forces are wanted, and
+// coefficients that the FMA reads from the constant bank.  Slots outside the
+// cutoff, padding and an atom with itself give any value, infinities and NaN
+// among them: the caller selects them away and must not multiply them by zero.
+// With an alpha rc beyond EWALD_Z_MAX (ewald_tol below 1e-6) the functions
+// themselves are called.  Pair launch at 100k atoms (half lists, energies)
 // 572 -> 392 us, forces alone 555 -> 330; 28k atoms 251 -> 155; 7,309 atoms
 // 178 -> 113; a batch of 64 small systems 1.92 -> 1.39 ms.
 template <bool POLY, bool ENERGY>

@@ -116,7 +116,7 @@ struct FFTPlan1D {
 
 // Buffers of mdf_backward, all in one allocation (Ctx::adj_mem): none is kept
 // from one call to the next, and a context's first gradient waits for one
-// cudaMalloc (3.6 -> 2.1 ms of a first training step at 28,000 atoms with nine).
+// cudaMalloc (first training step at 28,000 atoms 2.35 ms, with nine 3.4).
 struct AdjBufs {
     double* v;                             // [3N] dL/dF, atom order, normalised
     void* vs;                              // [slots] the same per slot (float4 or double4)

@@ -1,4 +1,4 @@
-// Nonbonded pair kernel and the FP64 excluded-pair / 1-4 kernels.
+// Nonbonded pair kernels (the excluded and 1-4 pairs: pair_terms.cuh).
 //
 // Replaces, in REFERENCE semantics:
 //   calculate_LJ_energy_pairlist     src/System/NonBondedEnergy.cpp:79-131
@@ -7,8 +7,7 @@
 //   calculate_EE_ewald_direct_term   :236-305
 //   calculate_forces_LJ_pairlist     src/System/NonBondedForces.cpp:92-155
 //   calculate_forces_EE_pairlist     src/System/NonBondedForces.cpp:207-241
-// and in PHYSICAL semantics the erfc real-space Ewald sum with switched LJ,
-// the excluded-pair erf corrections and the scaled 1-4 pairs.
+// and in PHYSICAL semantics the erfc real-space Ewald sum with switched LJ.
 //
 // Pair kernel layout: one warp per i cluster (8 atoms).  The warp walks the
 // cluster's half list four j clusters at a time; lane = (jslot, ii) with
@@ -787,8 +786,10 @@ __global__ void __launch_bounds__(NB_THREADS, 4) k_pairs_f32_force_multi(const P
 // offsets), the lane's mask row rotated once per entry, branch-free
 // selection of the inactive pairs, an (A, B, 12A, 6B) table in shared memory
 // and constants folded on the host.  The arithmetic differs only where
-// precision does: FP64 rsqrt, exp and erfc (the CUDA math library) instead of
-// the SFU forms and the A&S erfc, and FP64 image offsets from FP64 centres.
+// precision does: FP64 rsqrt instead of the SFU form, the Ewald terms as
+// polynomials in r^2 (ewald_f64; exp and erfc of the CUDA math library where
+// alpha and the cutoff lie beyond their range) instead of the A&S erfc, and FP64
+// image offsets from FP64 centres.
 template <bool ENERGY, bool SWITCH, bool COUNT, bool LJS, bool POLY>
 __device__ __forceinline__ void pairs_f64_body_t(SmemF64W& S, const PairF64Args& A, const EwaldPoly& T)
 {

@@ -424,10 +424,9 @@ constexpr int SEARCH_CAP = 512;   // entries a warp buffers (~125 per i cluster 
 // the buffer in pieces.  Entries past `cap` are counted but not written
 // (ST_CAPACITY_PAIRS: the host grows the list and searches again).
 //
-// Before, a lane walked whole columns alone, twice (count, write), and one warp
-// per excluded pair then searched its entry in global memory.
-// With the exclusions 100k atoms 245 -> 80 us, 960k 2,235 -> 730 us; a whole
-// build at 100k 336 -> 132 us, at 960k 2.56 -> 0.86 ms.
+// A lane per column, counting and then writing, and a warp per excluded pair that
+// searches its entry in global memory take 245 us where this takes 80 (100k
+// atoms; 960k 2,235 and 730; a whole build 336 and 132 us, 2.56 and 0.86 ms).
 __global__ void __launch_bounds__(32 * SEARCH_WARPS) k_pair_search(
     const int* __restrict__ d_ncl, const SearchGeom g, const int* __restrict__ cluster_col,
     const int* __restrict__ col_cstart, const float4* __restrict__ bb_lo, const float4* __restrict__ bb_hi,
@@ -618,11 +617,11 @@ __global__ void __launch_bounds__(32 * SEARCH_WARPS) k_pair_search(
 // minimum).
 //
 // What bounds it: gathers and latency (half the issue slots used, 470 warp
-// instructions per 32 entries).  One lane per entry with early exit, the form
-// before, read 32 lines per load instruction and three 16-byte box words per
-// entry; here a box is one 16-byte word and a test reads eight whole lines.
-// FP32 at 100k atoms 48 -> 44 us, at 960k 408 -> 359 us; FP64 half lists at
-// 100k (FP64 arithmetic before) 125 -> 50 us.  Loading the next 32 entries and
+// instructions per 32 entries).  One lane per entry with early exit reads 32
+// lines per load instruction and three 16-byte box words per entry; here a box is
+// one 16-byte word and a test reads eight whole lines.  FP32 at 100k atoms 44 us
+// against 48, at 960k 359 against 408; FP64 half lists at 100k 50 us against 125
+// with FP64 arithmetic.  Loading the next 32 entries and
 // boxes a round ahead gained nothing (42-52 us); at three blocks per SM,
 // without the 48 spilled bytes, 100k took 42 us but 960k 396 us.
 using F32x2 = unsigned long long;   // two packed FP32 values
