@@ -401,10 +401,11 @@ __device__ __forceinline__ bool excluded_entry(int I, int la, int a, int b, cons
     return true;
 }
 
-// Clusters beyond this extent (A) are pruned by the WIDE form; below it, whatever
-// the atoms move until the next build, the FP32 test's rounding stays near 1e-2
-// A^2.  Liquids stay at 5 to 10 A.
-constexpr float WIDE_EXTENT = 64.f;
+// Clusters beyond this extent (A) are pruned by the WIDE form.  Liquids stay at 5
+// to 10 A, and a slab that straddles the box edge at the vacuum beside it: with
+// a line at 64 A such a slab (100k atoms, 60 A of vacuum) took 64 us in the prune
+// instead of 43, 102 instead of 44 in FP64.
+constexpr float WIDE_EXTENT = 256.f;
 
 constexpr int SEARCH_WARPS = 4;
 constexpr int SEARCH_CAP = 512;   // entries a warp buffers (~125 per i cluster at liquid density, 10 + 2 A)
@@ -601,12 +602,12 @@ __global__ void __launch_bounds__(32 * SEARCH_WARPS) k_pair_search(
 // entry's exclusion mask (an entry whose only close pairs are excluded is
 // kept; the pair kernel applies the mask), so it keeps a superset of the exact
 // set, and it runs in FP32 in both precisions: |a - b|^2 = |a|^2 + |b|^2 - 2 a.b
-// rounds with the square of the clusters' extents, by ~1e-4 A^2 at liquid
-// density and ~2e-3 A^2 at half extents of 16 A (BoxF.fine), inside the radius'
-// 0.02 A margin (0.1 A^2 at a cutoff of 3 A).  Wider clusters, those of very
-// dilute systems, would lose pairs near the cutoff from extents of some hundred
-// A on: where there are some, their entries are tested without the expansion, in
-// the precision of the positions (WIDE, prune_wide).
+// rounds with the square of the clusters' extents, by at most 16 roundings of
+// |x|^2: ~1e-4 A^2 at liquid density and 0.05 A^2 at half extents of 128 A, inside
+// the radius' 0.02 A margin (0.4 A^2 at a cutoff of 10 A, 0.1 at 3 A).  Wider
+// clusters, those of very dilute systems, would lose pairs near the cutoff: where
+// there are some, their entries are tested without the expansion, in the
+// precision of the positions (WIDE, prune_wide).
 //
 // W warps share an i cluster (32 entries each per round).  An entry is first
 // tested lane by lane through the clusters' current boxes (k_pack): farther
@@ -733,7 +734,8 @@ __device__ __forceinline__ void prune_dev(const PruneArgs& A)
             k0 = todo && far2 < rc2 && A.box_fine && bi.fine && bj.fine;
             todo = todo && !k0;
         }
-        if (WIDE && todo && !(bi.fine && bj.fine)) {
+        if (WIDE && todo &&
+            fmaxf(fmaxf(fmaxf(bi.hx, bi.hy), fmaxf(bi.hz, bj.hx)), fmaxf(bj.hy, bj.hz)) > 0.5f * WIDE_EXTENT) {
             const float4 cJ = A.centerf[my.j];
             const float ox = -(((cI.x - cJ.x) - s6[0]) - s6[3]), oy = -(((cI.y - cJ.y) - s6[1]) - s6[4]),
                         oz = -(((cI.z - cJ.z) - s6[2]) - s6[5]);
