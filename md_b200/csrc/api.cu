@@ -359,17 +359,35 @@ void upload_topology(Ctx& c, const mdf_topology* t)
     c.excl_pairs.upload(ex.data(), ex.size(), s);
     c.excl_is14.upload(is14.data(), is14.size(), s);
     if (c.n_excl > 0) {
-        // the partners' rows behind their N + 1 offsets, in one upload
+        // the partners' rows behind their N + 1 offsets, in one upload; pairs of an
+        // atom with many partners go to a list of their own (EXCL_ROW_MAX)
+        std::vector<int> partners(c.N, 0), heavy;
+        for (int a : ex) ++partners[a];
+        const int longest = *std::max_element(partners.begin(), partners.end());
+        long long n_heavy = 0;
+        for (size_t i = 0; i < ex.size(); i += 2)
+            n_heavy += std::max(partners[ex[i]], partners[ex[i + 1]]) > EXCL_ROW_MAX;
+        const int row_max = n_heavy > EXCL_PAIRS_PER_PARTNER * longest ? longest : EXCL_ROW_MAX;
         std::vector<int> rows(c.N + 1 + ex.size(), 0);
-        int* nb = rows.data() + c.N + 1;
-        for (int a : ex) ++rows[a + 1];
+        for (size_t i = 0; i < ex.size(); i += 2) {
+            if (std::max(partners[ex[i]], partners[ex[i + 1]]) > row_max) {
+                heavy.insert(heavy.end(), {ex[i], ex[i + 1]});
+            } else {
+                ++rows[ex[i] + 1];
+                ++rows[ex[i + 1] + 1];
+            }
+        }
         for (int i = 0; i < c.N; ++i) rows[i + 1] += rows[i];
         std::vector<int> at(rows.begin(), rows.begin() + c.N);
+        int* nb = rows.data() + c.N + 1;
         for (size_t i = 0; i < ex.size(); i += 2) {
+            if (std::max(partners[ex[i]], partners[ex[i + 1]]) > row_max) continue;
             nb[at[ex[i]]++] = ex[i + 1];
             nb[at[ex[i + 1]]++] = ex[i];
         }
         c.ex_rows.upload(rows.data(), rows.size(), s);
+        c.n_ex_heavy = (int)(heavy.size() / 2);
+        if (c.n_ex_heavy > 0) c.ex_heavy.upload(heavy.data(), heavy.size(), s);
     }
     {
         std::vector<int> p(2 * (size_t)c.n_14);
@@ -839,7 +857,7 @@ void mdf_destroy(mdf_ctx* ctx)
     c.bond_atoms.release(); c.ub_atoms.release(); c.angle_atoms.release(); c.dih_atoms.release();
     c.imp_atoms.release(); c.cmap_atoms.release(); c.cmap_set.release(); c.bond_par.release(); c.ub_par.release();
     c.angle_par.release(); c.imp_par.release(); c.dih_par.release(); c.cmap_coeff.release();
-    c.excl_pairs.release(); c.pairs14.release(); c.p14_scale.release(); c.excl_is14.release(); c.ex_rows.release();
+    c.excl_pairs.release(); c.pairs14.release(); c.p14_scale.release(); c.excl_is14.release(); c.ex_rows.release(); c.ex_heavy.release();
     c.xyz.release(); c.atom_col.release(); c.col_count.release(); c.col_start.release(); c.col_cstart.release();
     c.col_atoms.release(); c.slot_atom.release(); c.atom_slot.release(); c.slot_type.release(); c.center.release(); c.centerf.release();
     c.bb_lo.release(); c.bb_hi.release(); c.xq_f.release(); c.xq_d.release(); c.cluster_col.release();

@@ -127,6 +127,17 @@ struct AdjBufs {
     void* cgrid;                           // its half-complex grid
 };
 
+// The pair search clears a cluster's excluded pairs in one warp, about 1.4 us per
+// partner of the longest row where few warps have any, 0.2 ns per pair where all
+// have; a warp per pair after the search takes 0.5 ns per pair.  Molecules stay
+// below EXCL_ROW_MAX partners (waters 2, proteins up to ~25) and a rigid body with
+// all its pairs excluded lies above: its pairs go to warps of their own, unless
+// there are more than EXCL_PAIRS_PER_PARTNER for each partner of the longest row.
+// 20,000 atoms: a body of 400 0.13 ms for the build, in the search 0.66; of 1,500
+// 0.70 and 2.27; 64 partners for every atom 0.43 and 0.22.
+constexpr int EXCL_ROW_MAX = 32;
+constexpr long long EXCL_PAIRS_PER_PARTNER = 2600;
+
 // --------------------------------------------------------------- context
 struct Ctx {
     int device = 0;
@@ -151,6 +162,8 @@ struct Ctx {
     DevBuf<double2> lj14AB;    // same indexing, 1-4 tables
     DevBuf<int> ljvalid;       // [(ntypes+1)^2] nb != 0
     DevBuf<int> ex_rows;       // each atom's excluded partners: N + 1 offsets, then the rows
+    DevBuf<int> ex_heavy;      // [2 n_ex_heavy] excluded pairs that the search leaves (EXCL_ROW_MAX)
+    int n_ex_heavy = 0;
     int hot_type[2] = {0, 0};  // the two most frequent atom types
     EwaldPoly ewald_poly{};    // FP64 PHYSICAL contexts
     int ntp = 0;               // ntypes + 1 (padding type appended)

@@ -595,6 +595,37 @@ __global__ void __launch_bounds__(32 * SEARCH_WARPS) k_pair_search(
     finish(held, done);
 }
 
+// Clear the mask bits of listed excluded pairs (those that the search left), a
+// warp per pair: its lanes scan the range of the pair's i cluster.
+__global__ void __launch_bounds__(256) k_exclusion_masks(int n, const int* __restrict__ pairs, const SearchGeom g,
+                                                         const int* __restrict__ atom_slot,
+                                                         const double* __restrict__ xyz,
+                                                         const double4* __restrict__ center,
+                                                         const ILRange* __restrict__ ilist, PairEntry* __restrict__ plist,
+                                                         long long cap)
+{
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (k >= n) return;
+    int a = pairs[2 * k], b = pairs[2 * k + 1];   // a < b
+    if (atom_slot[b] / CLUSTER < atom_slot[a] / CLUSTER) {
+        const int t = a;
+        a = b;
+        b = t;
+    }
+    const int I = atom_slot[a] / CLUSTER;
+    unsigned key;
+    int bit;
+    if (!excluded_entry(I, atom_slot[a] % CLUSTER, a, b, atom_slot, xyz, center, g.L, key, bit)) return;
+    const ILRange r = ilist[I];
+    const long long end = min((long long)r.start + r.count, cap);
+    for (long long e0 = r.start; e0 < end; e0 += 32) {
+        const long long e = e0 + lane;
+        const bool hit = e < end && plist[e].j == (int)(key >> 5) && plist[e].shift == (int)(key & 31u);
+        if (hit) atomicAnd(&plist[e].mask, ~(1ull << bit));
+        if (__any_sync(0xffffffffu, hit)) return;
+    }
+}
+
 // ------------------------------------------------------------- pruning
 // Dynamic pruning: keep the outer-list entries that have at least one atom
 // pair within the prune radius at the current positions, in list order, packed
@@ -1139,6 +1170,9 @@ void build_pairlist(Ctx& c)
                 d_ncl, g, c.cluster_col.p, c.col_cstart.p, c.bb_lo.p, c.bb_hi.p, c.center.p, c.slot_atom.p,
                 c.atom_slot.p, c.xyz.p, c.n_excl > 0 ? c.ex_rows.p : nullptr,
                 c.n_excl > 0 ? c.ex_rows.p + c.N + 1 : nullptr, c.d_build.p, c.plist.p, cap, c.ilist.p, c.status.p);
+            if (c.n_ex_heavy > 0)
+                k_exclusion_masks<<<grid_blocks(32LL * c.n_ex_heavy, th), th, 0, s>>>(
+                    c.n_ex_heavy, c.ex_heavy.p, g, c.atom_slot.p, c.xyz.p, c.center.p, c.ilist.p, c.plist.p, cap);
             MDF_CUDA_TRY(cudaGetLastError());
             MDF_CUDA_TRY(cudaMemcpyAsync(c.h_build, d_ncl, sizeof(int), cudaMemcpyDeviceToHost, s));
             MDF_CUDA_TRY(cudaMemcpyAsync(c.h_build + 1, c.d_build.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
