@@ -359,11 +359,11 @@ static void launch_term_args(const Ctx& c, const TermArgs& A, bool energy)
     if (A.gx == 0) return;
     const int th = 256;
     if (c.p.semantics == MDF_SEM_PHYSICAL) {
-        if (energy) k_terms<true, true><<<grid_of(A), th, 0, c.stream>>>(A);
-        else k_terms<true, false><<<grid_of(A), th, 0, c.stream>>>(A);
+        if (energy) launch_beside(c, k_terms<true, true>, grid_of(A), th, 0, A);
+        else launch_beside(c, k_terms<true, false>, grid_of(A), th, 0, A);
     } else {
-        if (energy) k_terms<false, true><<<grid_of(A), th, 0, c.stream>>>(A);
-        else k_terms<false, false><<<grid_of(A), th, 0, c.stream>>>(A);
+        if (energy) launch_beside(c, k_terms<false, true>, grid_of(A), th, 0, A);
+        else launch_beside(c, k_terms<false, false>, grid_of(A), th, 0, A);
     }
     MDF_CUDA_TRY(cudaGetLastError());
 }

@@ -70,6 +70,34 @@ struct PruneArgs {
     int force;
 };
 
+// Launch on the context's present stream of a kernel that runs beside its pair
+// kernel, asking for an L1 divided as the pair kernel divides it: 72% shared
+// memory with blocks of eight warps, all of it with smaller ones.  An SM has to
+// drain to change the division, and left to itself a kernel that needs little
+// shared memory gets little: where the pair kernel's blocks all fit on the chip at
+// once, the side streams' kernels then wait for it to end.  Unpruned mixed
+// evaluations back to back (with energies / forces alone): 20,400 atoms 168 / 205
+// us with the driver's choice, 140 / 145 with this; 27,600 179 / 216 and 139 / 159;
+// 100k pruned, two evaluations, 668 and 648; FP64 at 20,400 188 and 175; 2,800 the
+// same.  72% beside blocks of two or four warps costs 5-25%, 100% beside eight-warp
+// ones 1.5% from 100k atoms on.  A batch keeps the driver's choice (128 systems
+// 3.30 ms, 3.38 with 72%, 3.49 with 100%).
+template <typename... P, typename... A>
+void launch_beside(const Ctx& c, void (*kern)(P...), dim3 grid, int threads, size_t smem, A&&... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c.stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at.val.sharedMemCarveout = c.p.pair_warps == 2 || c.p.pair_warps == 4 ? 100 : 72;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    MDF_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
+}
+
 // ------------------------------------------------------------- pair kernels
 constexpr int WHOLE_LIST = 1 << 30;   // a list is one part (PairF32Args::part)
 

@@ -478,37 +478,37 @@ static dim3 grid_of_sets(const A& a, int sets)
     return g;
 }
 template <typename R>
-static void launch_z_r2c(const FFTZArgs<R>& A, size_t sm, cudaStream_t s, int sets = 1)
+static void launch_z_r2c(const Ctx& c, const FFTZArgs<R>& A, size_t sm, int sets = 1)
 {
     const dim3 g = grid_of_sets(A, sets);
-    if (A.d.r[0]) k_fftr_z_r2c<R><<<g, FFT_THREADS, sm, s>>>(A);
-    else k_fft_z_r2c<R><<<g, FFT_THREADS, sm, s>>>(A);
+    if (A.d.r[0]) launch_beside(c, k_fftr_z_r2c<R>, g, FFT_THREADS, sm, A);
+    else launch_beside(c, k_fft_z_r2c<R>, g, FFT_THREADS, sm, A);
 }
 template <typename R>
-static void launch_z_c2r(const FFTZArgs<R>& A, size_t sm, cudaStream_t s, int sets = 1)
+static void launch_z_c2r(const Ctx& c, const FFTZArgs<R>& A, size_t sm, int sets = 1)
 {
     const dim3 g = grid_of_sets(A, sets);
-    if (A.d.r[0]) k_fftr_z_c2r<R><<<g, FFT_THREADS, sm, s>>>(A);
-    else k_fft_z_c2r<R><<<g, FFT_THREADS, sm, s>>>(A);
+    if (A.d.r[0]) launch_beside(c, k_fftr_z_c2r<R>, g, FFT_THREADS, sm, A);
+    else launch_beside(c, k_fft_z_c2r<R>, g, FFT_THREADS, sm, A);
 }
 template <typename R>
-static void launch_y(const FFTYArgs<R>& A, size_t sm, cudaStream_t s, int sets = 1)
+static void launch_y(const Ctx& c, const FFTYArgs<R>& A, size_t sm, int sets = 1)
 {
     const dim3 g = grid_of_sets(A, sets);
-    if (!A.d.r[0]) k_fft_y<R><<<g, FFT_THREADS, sm, s>>>(A);
-    else if (A.inverse) k_fftr_y<R, true><<<g, FFT_THREADS, sm, s>>>(A);
-    else k_fftr_y<R, false><<<g, FFT_THREADS, sm, s>>>(A);
+    if (!A.d.r[0]) launch_beside(c, k_fft_y<R>, g, FFT_THREADS, sm, A);
+    else if (A.inverse) launch_beside(c, k_fftr_y<R, true>, g, FFT_THREADS, sm, A);
+    else launch_beside(c, k_fftr_y<R, false>, g, FFT_THREADS, sm, A);
 }
 template <typename R>
-static void launch_x_conv(const FFTXArgs<R>& A, bool energy, size_t sm, cudaStream_t s, int sets = 1)
+static void launch_x_conv(const Ctx& c, const FFTXArgs<R>& A, bool energy, size_t sm, int sets = 1)
 {
     const dim3 g = grid_of_sets(A, sets);
     if (A.d.r[0]) {
-        if (energy) k_fftr_x_conv<R, true><<<g, FFT_THREADS, sm, s>>>(A);
-        else k_fftr_x_conv<R, false><<<g, FFT_THREADS, sm, s>>>(A);
+        if (energy) launch_beside(c, k_fftr_x_conv<R, true>, g, FFT_THREADS, sm, A);
+        else launch_beside(c, k_fftr_x_conv<R, false>, g, FFT_THREADS, sm, A);
     } else {
-        if (energy) k_fft_x_conv<R, true><<<g, FFT_THREADS, sm, s>>>(A);
-        else k_fft_x_conv<R, false><<<g, FFT_THREADS, sm, s>>>(A);
+        if (energy) launch_beside(c, k_fft_x_conv<R, true>, g, FFT_THREADS, sm, A);
+        else launch_beside(c, k_fft_x_conv<R, false>, g, FFT_THREADS, sm, A);
     }
 }
 
@@ -1199,11 +1199,11 @@ template <typename R>
 static void conv_chain(Ctx& c, const PmeBufs<R>&, bool energy)
 {
     const FFTChain<R> F = make_fft_chain<R>(c, energy);
-    launch_z_r2c(F.zf, F.smz, c.stream);
-    launch_y(F.yf, F.smy, c.stream);
-    launch_x_conv(F.x, energy, F.smx, c.stream);
-    launch_y(F.yi, F.smy, c.stream);
-    launch_z_c2r(F.zi, F.smz, c.stream);
+    launch_z_r2c(c, F.zf, F.smz);
+    launch_y(c, F.yf, F.smy);
+    launch_x_conv(c, F.x, energy, F.smx);
+    launch_y(c, F.yi, F.smy);
+    launch_z_c2r(c, F.zi, F.smz);
 }
 
 // Many systems' FFT chains, one launch per pass (each struct array holds one
@@ -1294,7 +1294,7 @@ static void run_pme(Ctx& c, bool energy)
     const int th = 256;
     if (!ref) {
         const SpreadArgs S = make_spread_args(c);
-        if (S.s1 > S.s0) k_spread4_rows<R><<<grid_of(S), th, 0, c.stream>>>(S);
+        if (S.s1 > S.s0) launch_beside(c, k_spread4_rows<R>, grid_of(S), th, 0, S);
         if (distributed(c)) allreduce_u64(c, c.qgrid.p, ntot);   // the whole charge grid on every rank
     } else {
         k_spread_ref5<<<grid_blocks(c.N, th), th, 0, c.stream>>>(c.N, c.xyz.p, c.q.p, B.g, c.qgrid.p);
@@ -1304,7 +1304,7 @@ static void run_pme(Ctx& c, bool energy)
     mark(c, "pme_fft_conv");
     if (!ref) {
         const GatherArgs<R> G = make_gather_args<R>(c);
-        if (G.s1 > G.s0) k_gather4<R><<<grid_of(G), th, 0, c.stream>>>(G);
+        if (G.s1 > G.s0) launch_beside(c, k_gather4<R>, grid_of(G), th, 0, G);
     } else {
         c.forces_pme_ref.alloc(3 * (size_t)c.N);
         k_gather_ref5<<<grid_blocks(c.N, th), th, 0, c.stream>>>(c.N, c.xyz.p, c.q.p, B.g,
@@ -1441,7 +1441,7 @@ static void run_pme_slab(Ctx& c, bool energy)
         MDF_CUDA_TRY(cudaMemsetAsync(c.qgrid.p, 0, sizeof(unsigned long long) * (size_t)P * K0p * plane, c.stream));
     }
     const SpreadArgs S = make_spread_args(c);
-    if (S.s1 > S.s0) k_spread4_rows<R><<<grid_of(S), th, 0, c.stream>>>(S);
+    if (S.s1 > S.s0) launch_beside(c, k_spread4_rows<R>, grid_of(S), th, 0, S);
     MDF_CUDA_TRY(cudaGetLastError());
     if (halo) {
         // my slab = my own planes of my window + the planes other ranks spread into it
@@ -1481,18 +1481,18 @@ static void run_pme_slab(Ctx& c, bool energy)
     F.x.gy = ny;
     F.x.infl += (long long)r * K1p * Kc * K0;
     F.x.my += (long long)r * K1p;
-    launch_z_r2c(F.zf, F.smz, c.stream);
-    launch_y(F.yf, F.smy, c.stream);
+    launch_z_r2c(c, F.zf, F.smz);
+    launch_y(c, F.yf, F.smy);
     const int nb = (int)std::min<long long>(148 * 8, ((long long)P * blk + th - 1) / th);
     k_slab_to_blocks<C><<<nb, th, 0, c.stream>>>(slab, sendb, P, K0p, K1, K1p, Kc);
     MDF_CUDA_TRY(cudaGetLastError());
     coll_check(c.coll_a2a(sendb, recvb, (int64_t)(sizeof(C) * blk), (void*)c.stream, c.coll_user), "all-to-all");
-    if (ny > 0) launch_x_conv(F.x, energy, F.smx, c.stream);
+    if (ny > 0) launch_x_conv(c, F.x, energy, F.smx);
     // back: the x-pass layout [s][x][yl][kc] is already one block per rank
     coll_check(c.coll_a2a(recvb, sendb, (int64_t)(sizeof(C) * blk), (void*)c.stream, c.coll_user), "all-to-all");
     k_blocks_to_slab<C><<<nb, th, 0, c.stream>>>(sendb, slab, K0p, K1, K1p, Kc);
-    launch_y(F.yi, F.smy, c.stream);
-    launch_z_c2r(F.zi, F.smz, c.stream);
+    launch_y(c, F.yi, F.smy);
+    launch_z_c2r(c, F.zi, F.smz);
     MDF_CUDA_TRY(cudaGetLastError());
     if (halo) {
         // the potential of my slab in place, and of my window's other planes from their owners
@@ -1514,7 +1514,7 @@ static void run_pme_slab(Ctx& c, bool energy)
     }
     mark(c, "pme_fft_conv");
     const GatherArgs<R> G = make_gather_args<R>(c);
-    if (G.s1 > G.s0) k_gather4<R><<<grid_of(G), th, 0, c.stream>>>(G);
+    if (G.s1 > G.s0) launch_beside(c, k_gather4<R>, grid_of(G), th, 0, G);
     MDF_CUDA_TRY(cudaGetLastError());
     mark(c, "pme_gather");
     c.launches += 10;   // spread, z, y, pack, x+conv, unpack, y, z, gather (+ memset)
@@ -1716,11 +1716,11 @@ static void run_pme_adjoint(Ctx& c, double gE, const AdjBufs& M)
     F.zi.cgrid2 = F.zf.cgrid2;
     F.zi.rgrid2 = F.zf.rgrid2;
     F.yf.cgrid2 = F.yi.cgrid2 = F.x.cgrid2 = F.zf.cgrid2;
-    launch_z_r2c(F.zf, F.smz, c.stream, 2);
-    launch_y(F.yf, F.smy, c.stream, 2);
-    launch_x_conv(F.x, false, F.smx, c.stream, 2);
-    launch_y(F.yi, F.smy, c.stream, 2);
-    launch_z_c2r(F.zi, F.smz, c.stream, 2);
+    launch_z_r2c(c, F.zf, F.smz, 2);
+    launch_y(c, F.yf, F.smy, 2);
+    launch_x_conv(c, F.x, false, F.smx, 2);
+    launch_y(c, F.yi, F.smy, 2);
+    launch_z_c2r(c, F.zi, F.smz, 2);
     k_adj_gather<R><<<grid_blocks(c.n_slots, th), th, 0, c.stream>>>(
         c.n_slots, c.slot_atom.p, c.xyz.p, B.g, B.rg, F.zf.rgrid2, vs, gE, M.dq_slot, c.status.p);
     MDF_CUDA_TRY(cudaGetLastError());
